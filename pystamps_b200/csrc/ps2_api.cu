@@ -31,6 +31,7 @@
 #include "../../include/ps2cuda.h"
 #include "interp10_taps.h"
 #include "ps2_kernels.cuh"
+#include "v5_uniform.cuh"
 
 using namespace ps2;
 
@@ -83,66 +84,6 @@ struct DevBuf {
   }
   template <typename T>
   T* as() const { return static_cast<T*>(p); }
-};
-
-// MATLAB rand('state', seed) / v5 uniform generator (native_stage2.rs:1785-1873):
-// 32-word subtract-with-borrow lagged-Fibonacci state, xorshift-32 mantissa
-// scrambling of the 53-bit result.
-class V5Uniform {
- public:
-  explicit V5Uniform(uint32_t seed) : j_(seed == 0 ? (1u << 31) : seed) {
-    uint32_t s = j_;
-    for (int k = 0; k < 32; ++k) {
-      uint64_t x = 0;
-      for (int b = 0; b < 53; ++b) {
-        s = xs32(s);
-        x = (x << 1) | ((s >> 19) & 1u);
-      }
-      st_[k] = static_cast<double>(x) * kUlp;
-    }
-  }
-  double next() {
-    double v = st_[(ix_ + 20) & 31] - st_[(ix_ + 5) & 31] - borrow_;
-    if (v < 0.0) {
-      v += 1.0;
-      borrow_ = kUlp;
-    } else {
-      borrow_ = 0.0;
-    }
-    st_[ix_] = v;
-    ix_ = (ix_ + 1) & 31;
-    const uint32_t lo = j_, hi = xs32(lo);
-    j_ = hi;
-    const uint64_t mask = ((static_cast<uint64_t>(hi) << 32) & ((uint64_t(1) << 52) - 1)) ^ lo;
-    if (v == 0.0) return std::ldexp(static_cast<double>(mask), -53);
-    uint64_t bits;
-    std::memcpy(&bits, &v, 8);
-    const int eb = static_cast<int>((bits >> 52) & 0x7ff);
-    uint64_t mant = bits & ((uint64_t(1) << 52) - 1);
-    int ex;
-    if (eb == 0) {
-      const int lead = 63 - __builtin_clzll(mant);
-      ex = lead - 1073;
-      mant <<= (52 - lead);
-    } else {
-      ex = eb - 1022;
-      mant |= (uint64_t(1) << 52);
-    }
-    return std::ldexp(static_cast<double>(mant ^ mask), ex - 53);
-  }
-
- private:
-  static constexpr double kUlp = 1.1102230246251565e-16;  // 2^-53
-  static uint32_t xs32(uint32_t v) {
-    v ^= v << 13;
-    v ^= v >> 17;
-    v ^= v << 5;
-    return v;
-  }
-  double st_[32];
-  int ix_ = 0;
-  double borrow_ = 0.0;
-  uint32_t j_;
 };
 
 void coh_bin_rule(double* cutoff0, double* d) {
@@ -1582,19 +1523,29 @@ int ps2_random_coherence_histogram(const double* bperp_nm, int64_t n_ifg, double
     }
     cols = n_image;
   }
-  // random phases, column-major [cols][n_rand] (MATLAB draws the whole matrix first)
-  std::vector<double> rnd(static_cast<size_t>(n_rand) * cols);
-  {
-    V5Uniform rng(2005);
-    const double two_pi = 2.0 * M_PI;
-    for (auto& v : rnd) v = rng.next() * two_pi;
-  }
   Scoped sc;
   int rc = scoped_init(sc);
   if (rc) return rc;
-  DevBuf dr, db, dia, dib, dh;
-  CK(dr.alloc(sizeof(double) * rnd.size()));
-  CK(cudaMemcpyAsync(dr.p, rnd.data(), sizeof(double) * rnd.size(), cudaMemcpyHostToDevice, sc.st));
+  // random phases, column-major [cols][n_rand] (MATLAB draws the whole matrix
+  // first), drawn on the device
+  if (n_rand > (int64_t(1) << 40) / cols)
+    return set_err(PS2_ERR_OUT_OF_MEMORY, "ps2_random_coherence_histogram: %lld x %lld random phases", (long long)n_rand,
+                   (long long)cols);
+  const int64_t draws = n_rand * cols;
+  DevBuf dr, dtab, db, dia, dib, dh;
+  V5Tables tab;
+  v5_tables(draws, &tab);
+  const size_t b_step = sizeof(V5Num) * tab.step.size(), b_start = sizeof(V5Num) * tab.start.size();
+  CK(dr.alloc(sizeof(double) * draws));
+  CK(dtab.alloc(b_step + b_start + sizeof(uint32_t) * tab.jump.size()));
+  unsigned char* tabp = dtab.as<unsigned char>();
+  CK(cudaMemcpyAsync(tabp, tab.step.data(), b_step, cudaMemcpyHostToDevice, sc.st));
+  CK(cudaMemcpyAsync(tabp + b_step, tab.start.data(), b_start, cudaMemcpyHostToDevice, sc.st));
+  CK(cudaMemcpyAsync(tabp + b_step + b_start, tab.jump.data(), sizeof(uint32_t) * tab.jump.size(),
+                     cudaMemcpyHostToDevice, sc.st));
+  CK(launch_v5_uniform(reinterpret_cast<const V5Num*>(tabp), reinterpret_cast<const V5Num*>(tabp + b_step),
+                       reinterpret_cast<const uint32_t*>(tabp + b_step + b_start), 2.0 * M_PI, dr.as<double>(), draws,
+                       sc.st));
   CK(db.alloc(sizeof(double) * n_ifg));
   CK(cudaMemcpyAsync(db.p, bperp_nm, sizeof(double) * n_ifg, cudaMemcpyHostToDevice, sc.st));
   CK(dia.alloc(sizeof(int64_t) * n_ifg));
