@@ -58,27 +58,155 @@ int set_err(int code, const char* fmt, ...) {
     }                                                                                                         \
   } while (0)
 
-// Device allocation owned by a context.
+// Device blocks and streams that calls and contexts hand back, kept for the next
+// one. A call over host rows, or the load of a small patch, spent most of its
+// time in cudaMalloc, cudaFree and stream creation (5 to 30 ms of 7 to 100 ms,
+// against 0.2 to 5 ms of device work). Kept per device: at most kMaxBytes in
+// blocks of at most kMaxBlock bytes (a full-scale patch's arrays, a few GB, go
+// back to the driver) and at most kMaxStreams idle streams; an allocation that
+// fails first gives every kept block back; a mutex guards the lists. A block
+// enters the cache only where the calling thread has named the one stream its
+// work runs on (CallStream) and that stream has been waited for; any other block
+// is freed by cudaFree, which waits for the whole device.
+thread_local cudaStream_t g_call_stream = nullptr;
+struct CallStream {
+  cudaStream_t before;
+  explicit CallStream(cudaStream_t s) : before(g_call_stream) { g_call_stream = s; }
+  CallStream(const CallStream&) = delete;
+  CallStream& operator=(const CallStream&) = delete;
+  ~CallStream() { g_call_stream = before; }
+};
+class DeviceCache {
+ public:
+  static constexpr size_t kMaxBytes = size_t(512) << 20, kMaxBlock = size_t(384) << 20;
+  static constexpr size_t kMaxStreams = 16;
+  static constexpr int kMaxDevices = 64;
+
+  static DeviceCache& get() {
+    static DeviceCache* c = new DeviceCache();  // never destroyed: the driver may end before static objects do
+    return *c;
+  }
+  // Blocks are rounded up to 1/8 of their power of two (512 bytes at least), and
+  // a kept block serves requests down to 3/4 of its size: waste stays below a third.
+  static size_t rounded(size_t n) {
+    size_t g = 512;
+    while (g * 16 <= n) g *= 2;
+    return (n + g - 1) / g * g;
+  }
+  cudaError_t alloc(void** p, size_t* bytes, int* device) {
+    const size_t want = rounded(*bytes);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    *device = dev;
+    if (dev < kMaxDevices) {
+      std::lock_guard<std::mutex> g(mu_);
+      auto& l = blocks_[dev];
+      size_t best = l.size();
+      for (size_t i = 0; i < l.size(); ++i)
+        if (l[i].second >= want && l[i].second - l[i].second / 4 <= want &&
+            (best == l.size() || l[i].second < l[best].second))
+          best = i;
+      if (best < l.size()) {
+        *p = l[best].first;
+        *bytes = l[best].second;
+        held_[dev] -= *bytes;
+        l[best] = l.back();
+        l.pop_back();
+        return cudaSuccess;
+      }
+    }
+    e = cudaMalloc(p, want);
+    if (e == cudaErrorMemoryAllocation && dev < kMaxDevices) {
+      cudaGetLastError();
+      give_back(dev);
+      e = cudaMalloc(p, want);
+    }
+    if (e == cudaSuccess) *bytes = want;
+    return e;
+  }
+  void release(void* p, size_t bytes, int device) {
+    int dev = 0;
+    if (g_call_stream && bytes <= kMaxBlock && cudaGetDevice(&dev) == cudaSuccess && dev == device &&
+        dev < kMaxDevices && cudaStreamSynchronize(g_call_stream) == cudaSuccess) {
+      std::lock_guard<std::mutex> g(mu_);
+      if (held_[dev] + bytes <= kMaxBytes) {
+        blocks_[dev].emplace_back(p, bytes);
+        held_[dev] += bytes;
+        return;
+      }
+    }
+    cudaFree(p);
+  }
+  cudaError_t stream(cudaStream_t* s) {
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    if (dev < kMaxDevices) {
+      std::lock_guard<std::mutex> g(mu_);
+      if (!streams_[dev].empty()) {
+        *s = streams_[dev].back();
+        streams_[dev].pop_back();
+        return cudaSuccess;
+      }
+    }
+    return cudaStreamCreateWithFlags(s, cudaStreamNonBlocking);
+  }
+  void release(cudaStream_t s) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess && dev < kMaxDevices && cudaStreamSynchronize(s) == cudaSuccess) {
+      std::lock_guard<std::mutex> g(mu_);
+      if (streams_[dev].size() < kMaxStreams) {
+        streams_[dev].push_back(s);
+        return;
+      }
+    }
+    cudaStreamDestroy(s);
+  }
+
+ private:
+  void give_back(int dev) {
+    std::vector<std::pair<void*, size_t>> all;
+    {
+      std::lock_guard<std::mutex> g(mu_);
+      all.swap(blocks_[dev]);
+      held_[dev] = 0;
+    }
+    for (auto& b : all) cudaFree(b.first);
+  }
+  std::mutex mu_;
+  std::vector<std::pair<void*, size_t>> blocks_[kMaxDevices];
+  std::vector<cudaStream_t> streams_[kMaxDevices];
+  size_t held_[kMaxDevices] = {};
+};
+
+// Device allocation owned by a context or a call.
 struct DevBuf {
   void* p = nullptr;
   size_t bytes = 0;
+  int device = 0;
+  bool direct = false;  // used on a caller's stream: never cached
   DevBuf() = default;
   DevBuf(const DevBuf&) = delete;
   DevBuf& operator=(const DevBuf&) = delete;
   ~DevBuf() { release(); }
   // keeps the current allocation when it is large enough (a context reloads
-  // patches without returning to cudaMalloc/cudaFree, which synchronise)
+  // patches without returning to the allocator, which synchronises)
   cudaError_t alloc(size_t n) {
     if (n == 0) n = 16;
     if (p && bytes >= n) return cudaSuccess;
     release();
-    cudaError_t e = cudaMalloc(&p, n);
-    if (e == cudaSuccess) bytes = n;
+    size_t got = n;
+    cudaError_t e = DeviceCache::get().alloc(&p, &got, &device);
+    if (e == cudaSuccess) bytes = got;
     else p = nullptr;
     return e;
   }
   void release() {
-    if (p) cudaFree(p);
+    if (p && direct)
+      cudaFree(p);
+    else if (p)
+      DeviceCache::get().release(p, bytes, device);
     p = nullptr;
     bytes = 0;
   }
@@ -217,6 +345,20 @@ struct ps2_ctx {
 };
 
 namespace {
+
+std::vector<DevBuf*> context_buffers(ps2_ctx* c) {
+  return {&c->ph_nm, &c->bp, &c->amp, &c->perm, &c->cell_start, &c->cell_of, &c->w0, &c->K[0], &c->K[1], &c->w, &c->coh,
+          &c->C, &c->nopt, &c->grid, &c->win, &c->wpart, &c->filt, &c->low_pass, &c->wscaled, &c->taps, &c->lut, &c->nr0,
+          &c->nr_scaled, &c->state, &c->stats, &c->hist, &c->n_invalid, &c->rms_partial, &c->ph_res, &c->scratch,
+          &c->stage, &c->stage_bp, &c->bt, &c->ad_ph, &c->ad_K, &c->ad_w, &c->ad_coh, &c->ad_grid, &c->ad_win,
+          &c->ad_filt, &c->ad_gfilt, &c->ad_gph, &c->ad_gK, &c->ad_gf, &c->ad_part};
+}
+
+// From here on work on a stream that is not the context's own may read its
+// buffers: they go back through cudaFree.
+void mark_foreign(ps2_ctx* c) {
+  for (DevBuf* b : context_buffers(c)) b->direct = true;
+}
 
 size_t rsz(const ps2_ctx* c) { return c->fp64 ? sizeof(double) : sizeof(float); }
 size_t csz(const ps2_ctx* c) { return 2 * rsz(c); }
@@ -537,17 +679,11 @@ int ps2_create(ps2_ctx** out, int device) {
   CK(cudaSetDevice(device));
   ps2_ctx* c = new ps2_ctx();
   c->device = device;
-  cudaDeviceProp prop;
-  cudaError_t e = cudaGetDeviceProperties(&prop, device);
-  if (e != cudaSuccess) {
-    delete c;
-    return set_err(PS2_ERR_CUDA, "cudaGetDeviceProperties: %s", cudaGetErrorString(e));
-  }
-  c->sm_count = prop.multiProcessorCount;
-  e = cudaStreamCreateWithFlags(&c->st, cudaStreamNonBlocking);
+  cudaError_t e = cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, device);
+  if (e == cudaSuccess) e = DeviceCache::get().stream(&c->st);
   if (e == cudaSuccess) e = cudaMallocHost(reinterpret_cast<void**>(&c->h_stats), 8 * sizeof(double));
   if (e != cudaSuccess) {
-    if (c->st) cudaStreamDestroy(c->st);
+    if (c->st) DeviceCache::get().release(c->st);
     delete c;
     return set_err(PS2_ERR_CUDA, "ps2_create: %s", cudaGetErrorString(e));
   }
@@ -562,24 +698,18 @@ void ps2_destroy(ps2_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   if (c->st) cudaStreamSynchronize(c->st);
-  DevBuf* bufs[] = {&c->ph_nm, &c->bp, &c->amp, &c->perm, &c->cell_start, &c->cell_of, &c->w0, &c->K[0], &c->K[1],
-                    &c->w, &c->coh, &c->C, &c->nopt, &c->grid, &c->win, &c->wpart, &c->filt, &c->low_pass, &c->wscaled,
-                    &c->taps, &c->lut, &c->nr0, &c->nr_scaled, &c->state, &c->stats, &c->hist, &c->n_invalid,
-                    &c->rms_partial, &c->ph_res, &c->scratch, &c->stage, &c->ad_ph, &c->ad_K, &c->ad_w,
-                    &c->ad_coh, &c->ad_grid, &c->ad_win, &c->ad_filt, &c->ad_gfilt, &c->ad_gph, &c->ad_gK,
-                    &c->ad_gf, &c->ad_part};
-  for (DevBuf* b : bufs) b->release();
+  CallStream call(c->st);
+  if (c->cst) cudaStreamSynchronize(c->cst);
+  for (DevBuf* b : context_buffers(c)) b->release();
   drop_loop_graph(c);
   for (cudaEvent_t e : c->evpool) cudaEventDestroy(e);
   if (c->ad_ev) cudaEventDestroy(c->ad_ev);
-  c->stage_bp.release();
   if (c->ev_ph) cudaEventDestroy(c->ev_ph);
   if (c->ev_bp) cudaEventDestroy(c->ev_bp);
-  if (c->cst) cudaStreamDestroy(c->cst);
-  c->bt.release();
+  if (c->cst) DeviceCache::get().release(c->cst);
   if (c->h_active) cudaFreeHost(c->h_active);
   if (c->h_stats) cudaFreeHost(c->h_stats);
-  if (c->st) cudaStreamDestroy(c->st);
+  if (c->st) DeviceCache::get().release(c->st);
   delete c;
 }
 
@@ -635,10 +765,11 @@ int ps2_load_patch(ps2_ctx* c, const ps2_patch_desc* d) {
   // transfer overlaps the host's cell sort; the gathers below wait for them.
   // Every return from here on waits for these copies (the caller's buffers are
   // not kept past the call).
-  if (!c->cst) CK(cudaStreamCreateWithFlags(&c->cst, cudaStreamNonBlocking));
+  if (!c->cst) CK(DeviceCache::get().stream(&c->cst));
   if (!c->ev_ph) CK(cudaEventCreateWithFlags(&c->ev_ph, cudaEventDisableTiming));
   if (!c->ev_bp) CK(cudaEventCreateWithFlags(&c->ev_bp, cudaEventDisableTiming));
   CK(cudaStreamSynchronize(c->st));
+  CallStream call(c->st);
   struct CopyJoin {
     cudaStream_t s;
     ~CopyJoin() { cudaStreamSynchronize(s); }
@@ -748,6 +879,11 @@ int ps2_load_patch(ps2_ctx* c, const ps2_patch_desc* d) {
   CK(c->nr_scaled.alloc(sizeof(double) * PS2_COH_BINS));
   CK(c->state.alloc(sizeof(double) * 4));
   CK(c->stats.alloc(sizeof(double) * 8));
+  // a block may hold an earlier owner's data: what a download before the first
+  // iteration reads starts at zero
+  CK(cudaMemsetAsync(c->C.p, 0, R * N, c->st));
+  CK(cudaMemsetAsync(c->nopt.p, 0, N, c->st));
+  CK(cudaMemsetAsync(c->stats.p, 0, sizeof(double) * 8, c->st));
   CK(c->hist.alloc(sizeof(int32_t) * PS2_COH_BINS));
   CK(c->n_invalid.alloc(sizeof(int32_t)));
   c->topo_blocks = topofit_grid_blocks(c->sm_count, c->fp64);
@@ -958,6 +1094,7 @@ int ps2_import_state(ps2_ctx* c, const void* buf, int64_t bytes) {
 int ps2_autotune(ps2_ctx* c, int32_t* chosen_lanes, double* ms_per_candidate) {
   if (!c || !c->loaded) return set_err(PS2_ERR_NOT_LOADED, "no patch loaded");
   CK(cudaSetDevice(c->device));
+  CallStream call(c->st);
   int rc = ensure_events(c, 2);
   if (rc) return rc;
   auto timed = [&](auto&& launch, double* ms_out) -> int {
@@ -1097,6 +1234,7 @@ int ps2_download(ps2_ctx* c, ps2_outputs* o) {
   if (!c || !c->loaded) return set_err(PS2_ERR_NOT_LOADED, "no patch loaded");
   if (!o) return set_err(PS2_ERR_INVALID_ARG, "NULL outputs");
   CK(cudaSetDevice(c->device));
+  CallStream call(c->st);
   const int64_t N = c->N, M = c->M, G = c->G;
   const size_t R = rsz(c), Cz = csz(c);
   const int32_t* perm = c->perm.as<int32_t>();
@@ -1219,17 +1357,23 @@ namespace {
 struct Scoped {
   cudaStream_t st = nullptr;
   int sm = 148;
+  cudaStream_t before = nullptr;
+  // declared ahead of the call's buffers: they are released first, into the
+  // cache once the stream is idle
   ~Scoped() {
-    if (st) cudaStreamDestroy(st);
+    if (!st) return;
+    g_call_stream = before;
+    DeviceCache::get().release(st);
   }
 };
+// One attribute, not cudaGetDeviceProperties: that query alone took 5 to 28 ms.
 int scoped_init(Scoped& s) {
   int dev;
   CK(cudaGetDevice(&dev));
-  cudaDeviceProp p;
-  CK(cudaGetDeviceProperties(&p, dev));
-  s.sm = p.multiProcessorCount;
-  CK(cudaStreamCreateWithFlags(&s.st, cudaStreamNonBlocking));
+  CK(cudaDeviceGetAttribute(&s.sm, cudaDevAttrMultiProcessorCount, dev));
+  CK(DeviceCache::get().stream(&s.st));
+  s.before = g_call_stream;
+  g_call_stream = s.st;
   return PS2_OK;
 }
 }  // namespace
@@ -1722,6 +1866,7 @@ int coh_check(ps2_ctx* c, const void* a, const void* b, const void* d, double al
 int coh_prologue(ps2_ctx* c, const float* d_ph, const float* d_K, const float* d_w, double alpha, double beta,
                  cudaStream_t st, ClapArgs* ca_out) {
   CK(cudaSetDevice(c->device));
+  mark_foreign(c);
   // the patch upload and any loop work run on the context's stream: order after them
   if (!c->ad_ev) CK(cudaEventCreateWithFlags(&c->ad_ev, cudaEventDisableTiming));
   CK(cudaEventRecord(c->ad_ev, c->st));
@@ -1906,6 +2051,13 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   }
   CK(cudaSetDevice(c0->device));
   cudaStream_t st = c0->st;
+  CallStream call(st);
+  // every return waits for the batch's work: no context's buffers are in use on
+  // this stream after the call
+  struct BatchJoin {
+    cudaStream_t s;
+    ~BatchJoin() { cudaStreamSynchronize(s); }
+  } join{st};
   int rc = ensure_events(c0, 2);
   if (rc) return rc;
   // start after every patch's own queued work (its upload)
@@ -2163,14 +2315,10 @@ int ps3_reestimate(const ps3_reestimate_desc* d, ps3_reestimate_out* o, int devi
   if (rc) return rc;
   const int64_t n_jobs = static_cast<int64_t>(jobs.size() / 4);
   std::vector<int32_t> fit(d->fit_ifg, d->fit_ifg + d->n_fit);
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, device));
-  cudaStream_t st;
-  CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-  struct StreamGuard {
-    cudaStream_t s;
-    ~StreamGuard() { cudaStreamDestroy(s); }
-  } guard{st};
+  Scoped sc;
+  rc = scoped_init(sc);
+  if (rc) return rc;
+  cudaStream_t st = sc.st;
   DevBuf grid, ph, bp, djobs, djob_of, jout, dfit, lp, pp2, K2, C2, coh2, res2;
   const size_t gbytes = sizeof(float2) * d->grid_rows * d->grid_cols * M;
   CK(grid.alloc(gbytes));
@@ -2211,7 +2359,7 @@ int ps3_reestimate(const ps3_reestimate_desc* d, ps3_reestimate_out* o, int devi
   ca.low_pass = lp.as<double>();
   gauss7(ca.g7, nullptr);
   ca.job_out = jout.as<float2>();
-  CK(launch_s3_clap(ca, tf, prop.multiProcessorCount, st));
+  CK(launch_s3_clap(ca, tf, sc.sm, st));
   S3FitArgs fa{};
   fa.ph = ph.as<float2>();
   fa.bp = bp.as<float>();
@@ -2232,7 +2380,7 @@ int ps3_reestimate(const ps3_reestimate_desc* d, ps3_reestimate_out* o, int devi
   fa.C2 = C2.as<double>();
   fa.coh2 = coh2.as<double>();
   fa.ph_res2 = res2.as<float>();
-  CK(launch_s3_fit(fa, prop.multiProcessorCount, st));
+  CK(launch_s3_fit(fa, sc.sm, st));
   CK(cudaMemcpyAsync(o->ph_patch2, pp2.p, sizeof(float2) * n * M, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(o->ph_res2, res2.p, sizeof(float) * n * M, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(o->K_ps2, K2.p, sizeof(double) * n, cudaMemcpyDeviceToHost, st));
@@ -2284,6 +2432,7 @@ int ps2_stage3_reestimate(ps2_ctx* c, const int64_t* sel, int64_t n_sel, const i
     return set_err(PS2_ERR_UNSUPPORTED, "ps2_stage3_reestimate: %lld fit interferograms x %d trials exceed shared memory",
                    (long long)n_fit, 2 * n_half + 1);
   cudaStream_t st = c->st;
+  CallStream call(st);
   DevBuf djobs, djob_of, drow, dfit, jout, pp2, K2, C2, coh2, res2;
   CK(djobs.alloc(sizeof(int32_t) * jobs.size()));
   CK(cudaMemcpyAsync(djobs.p, jobs.data(), sizeof(int32_t) * jobs.size(), cudaMemcpyHostToDevice, st));
