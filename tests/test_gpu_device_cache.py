@@ -53,3 +53,27 @@ def test_context_in_used_blocks(cuda_lib):
     np.testing.assert_array_equal(before["C_ps"], again["C_ps"])
     for k in keys:
         np.testing.assert_array_equal(first[k], second[k])
+
+
+def test_download_vectors_are_not_overwritten(cuda_lib):
+    """The context hands out its result memory again only when no vector of an
+    earlier download is left."""
+    from pystamps_b200 import stage2 as S
+    from pystamps_b200 import synth
+
+    p = S.prepare_patch(synth.make_patch(2000, 12, 26, 41, seed=6, gamma_max_iterations=2))
+    with S.Stage2Context() as c:
+        c.load(p, "fp32")
+        c.iterate(1)
+        first = c.download(("K_ps", "coh_ps"))
+        kept, tail = first["K_ps"].copy(), first["coh_ps"][7:]
+        tail_kept = tail.copy()
+        c.iterate(1)
+        second = c.download(("K_ps", "coh_ps"))
+        assert not np.array_equal(first["K_ps"], second["K_ps"])
+        np.testing.assert_array_equal(first["K_ps"], kept)
+        del first, second  # `tail` still refers to the first download's memory
+        third = c.download(("K_ps", "coh_ps", "C_ps"))
+        np.testing.assert_array_equal(tail, tail_kept)
+        assert all(v.flags.c_contiguous and v.flags.writeable and v.shape == (2000,) for v in
+                   (third["K_ps"], third["coh_ps"], third["C_ps"]))
