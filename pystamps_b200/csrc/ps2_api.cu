@@ -393,6 +393,19 @@ BinArgs bin_args(ps2_ctx* c, int mode, const void* K) {
   return a;
 }
 
+BeginArgs begin_args(ps2_ctx* c, bool later) {
+  BeginArgs a{};
+  a.bin = bin_args(c, 0, c->K[0].p);
+  a.K1 = c->K[1].p;
+  a.N = c->N;
+  a.weights = later && c->psquare ? 1 : 0;
+  a.hist = c->hist.as<int32_t>();
+  a.n_invalid = c->n_invalid.as<int32_t>();
+  a.rms_partial = c->rms_partial.as<double>();
+  a.n_partial = c->topo_blocks;
+  return a;
+}
+
 ClapArgs clap_args(ps2_ctx* c, const void* grid, void* win) {
   ClapArgs a{};
   a.grid = grid;
@@ -522,8 +535,10 @@ FinalizeArgs finalize_args(ps2_ctx* c, bool force_continue) {
 
 // Queues one gamma iteration on the context's stream. `later` selects the form
 // of iterations 2.. (P-square weights from the previous table, or the SNR
-// weight kernel); `capturing` queues into a graph without touching counters.
-int enqueue_iteration(ps2_ctx* c, bool later, bool force_continue, cudaEvent_t* ev, int64_t* launched_out) {
+// weight kernel); `loop` is the condition of the WHILE node whose body this
+// iteration is captured into.
+int enqueue_iteration(ps2_ctx* c, bool later, bool force_continue, cudaEvent_t* ev, int64_t* launched_out,
+                      const cudaGraphConditionalHandle* loop = nullptr) {
   const bool fp64 = c->fp64;
   int64_t launched = 0;
   if (ev) CK(cudaEventRecord(ev[0], c->st));
@@ -533,14 +548,8 @@ int enqueue_iteration(ps2_ctx* c, bool later, bool force_continue, cudaEvent_t* 
     CK(launch_snr_weight(t, c->amp.as<float>(), c->w.p, fp64, c->sm_count, c->st));
     ++launched;
   }
-  CK(cudaMemsetAsync(c->hist.p, 0, sizeof(int32_t) * PS2_COH_BINS, c->st));
-  CK(cudaMemsetAsync(c->n_invalid.p, 0, sizeof(int32_t), c->st));
-  CK(cudaMemsetAsync(c->rms_partial.p, 0, sizeof(double) * c->topo_blocks, c->st));
-  if (later && c->psquare) {
-    // the P-square weights of this iteration, then binning with them (mode 0)
-    CK(launch_psquare_weights(bin_args(c, 1, c->K[0].p), c->N, fp64, c->sm_count, c->st));
-    ++launched;
-  }
+  CK(launch_iter_begin(begin_args(c, later), fp64, c->sm_count, c->st));
+  ++launched;
   CK(launch_bin(bin_args(c, 0, c->K[0].p), fp64, c->sm_count, c->st));
   ++launched;
   if (ev) CK(cudaEventRecord(ev[1], c->st));
@@ -550,15 +559,19 @@ int enqueue_iteration(ps2_ctx* c, bool later, bool force_continue, cudaEvent_t* 
   CK(launch_overlap(ov, fp64, c->st));
   launched += 2;
   if (ev) CK(cudaEventRecord(ev[2], c->st));
-  // K[1] keeps the K this iteration binned with (pm1's ph_weight needs it);
-  // topofit then rewrites K[0] in place
-  CK(cudaMemcpyAsync(c->K[1].p, c->K[0].p, rsz(c) * c->N, cudaMemcpyDeviceToDevice, c->st));
+  // rewrites K[0] in place; K[1] keeps the K this iteration binned with (pm1's
+  // ph_weight needs it)
   TopoArgs t = topo_args(c, c->K[0].p, c->C.p, c->coh.p);
   if (!c->psquare) t.ph_res = c->ph_res.p;
   CK(launch_topofit(t, fp64, c->topo_blocks, c->st));
   ++launched;
   if (ev) CK(cudaEventRecord(ev[3], c->st));
-  CK(launch_finalize(finalize_args(c, force_continue), c->st));
+  FinalizeArgs f = finalize_args(c, force_continue);
+  if (loop) {
+    f.set_loop = 1;
+    f.loop = *loop;
+  }
+  CK(launch_finalize(f, c->st));
   ++launched;
   if (ev) CK(cudaEventRecord(ev[4], c->st));
   if (launched_out) *launched_out = launched;
@@ -582,8 +595,8 @@ void drop_loop_graph(ps2_ctx* c) {
 }
 
 // The loop from iteration 2 on as one graph: a WHILE conditional node whose
-// body is one iteration followed by k_loop_continue, which clears the
-// condition when finalize raised the stop flag (native_stage2.rs:312-314).
+// body is one iteration; its k_finalize clears the condition when it raises the
+// stop flag (native_stage2.rs:312-314).
 int build_loop_graph(ps2_ctx* c, int64_t* body_launches) {
   cudaGraph_t g = nullptr;
   CK(cudaGraphCreate(&g, 0));
@@ -600,15 +613,13 @@ int build_loop_graph(ps2_ctx* c, int64_t* body_launches) {
   cudaGraph_t body = p.conditional.phGraph_out[0];
   CK(cudaStreamBeginCaptureToGraph(c->st, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
   int64_t launched = 0;
-  int rc = enqueue_iteration(c, true, false, nullptr, &launched);
-  cudaError_t e2 = rc ? cudaSuccess : launch_loop_continue(h, c->stats.as<double>(), c->st);
+  int rc = enqueue_iteration(c, true, false, nullptr, &launched, &h);
   cudaGraph_t captured = nullptr;
   cudaError_t e3 = cudaStreamEndCapture(c->st, &captured);
   if (rc) return rc;
-  CK(e2);
   CK(e3);
   CK(cudaGraphInstantiate(&c->loop_exec, g, 0));
-  *body_launches = launched + 1;
+  *body_launches = launched;
   return PS2_OK;
 }
 
@@ -2019,7 +2030,7 @@ namespace {
 // device image of a batch, laid out in one allocation
 struct BatchPlan {
   std::vector<PatchDev> patch;
-  std::vector<int64_t> bin_prefix, clap_prefix, ov_prefix;
+  std::vector<int64_t> bin_prefix, clap_prefix, ov_prefix, ps_prefix;
   std::vector<int32_t> units[4];  // (patch, virtual block) pairs per lane class 4, 8, 16, 32
   size_t smem_max[4] = {0, 0, 0, 0};
 };
@@ -2072,6 +2083,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   plan.bin_prefix.assign(1, 0);
   plan.clap_prefix.assign(1, 0);
   plan.ov_prefix.assign(1, 0);
+  plan.ps_prefix.assign(1, 0);
   int64_t cap_iter = 1;
   for (int64_t p = 0; p < n; ++p) {
     ps2_ctx* c = ctxs[p];
@@ -2100,6 +2112,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
                                              : static_cast<int64_t>(c->nwi) * c->nwj;
     plan.clap_prefix.push_back(plan.clap_prefix.back() + clap_units * (c->Mp / 4));
     plan.ov_prefix.push_back(plan.ov_prefix.back() + c->G * c->Mp);
+    plan.ps_prefix.push_back(plan.ps_prefix.back() + c->N);
     cap_iter = std::max<int64_t>(cap_iter, std::max<int64_t>(c->max_iter, 1) + 1);
   }
   // one device allocation: patches | active | n_active | prefixes | unit lists
@@ -2107,7 +2120,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   const size_t o_active = align256(o_patch + sizeof(PatchDev) * n);
   const size_t o_nact = align256(o_active + sizeof(int) * n);
   const size_t o_pref = align256(o_nact + sizeof(int));
-  const size_t o_units = align256(o_pref + sizeof(int64_t) * 3 * (n + 1));
+  const size_t o_units = align256(o_pref + sizeof(int64_t) * 4 * (n + 1));
   size_t o_cls[4], end = o_units;
   for (int k = 0; k < 4; ++k) {
     o_cls[k] = end;
@@ -2121,6 +2134,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   std::memcpy(pref, plan.bin_prefix.data(), sizeof(int64_t) * (n + 1));
   std::memcpy(pref + (n + 1), plan.clap_prefix.data(), sizeof(int64_t) * (n + 1));
   std::memcpy(pref + 2 * (n + 1), plan.ov_prefix.data(), sizeof(int64_t) * (n + 1));
+  std::memcpy(pref + 3 * (n + 1), plan.ps_prefix.data(), sizeof(int64_t) * (n + 1));
   for (int k = 0; k < 4; ++k)
     if (!plan.units[k].empty())
       std::memcpy(img.data() + o_cls[k], plan.units[k].data(), sizeof(int32_t) * plan.units[k].size());
@@ -2136,13 +2150,14 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   b.bin_prefix = reinterpret_cast<const int64_t*>(base + o_pref);
   b.clap_prefix = b.bin_prefix + (n + 1);
   b.ov_prefix = b.bin_prefix + 2 * (n + 1);
+  b.ps_prefix = b.bin_prefix + 3 * (n + 1);
   std::vector<int64_t> before(static_cast<size_t>(n));
   for (int64_t p = 0; p < n; ++p) before[p] = ctxs[p]->last.i_loop;
   const int lanes_of[4] = {4, 8, 16, 32};
-  int per_iter = 5;  // reset, bin, clap, overlap, finalize + one topofit per lane class
+  int per_iter = 5;  // begin, bin, clap, overlap, finalize + one topofit per lane class
   for (int cls = 0; cls < 4; ++cls) per_iter += plan.units[cls].empty() ? 0 : 1;
   auto enqueue = [&]() -> int {
-    CK(launch_batch_reset(b, st));
+    CK(launch_batch_begin(b, plan.ps_prefix.back(), c0->sm_count, st));
     CK(launch_batch_bin(b, plan.bin_prefix.back(), c0->sm_count, st));
     CK(launch_batch_clap(b, plan.clap_prefix.back(), c0->twf, c0->sm_count, st));
     CK(launch_batch_overlap(b, plan.ov_prefix.back(), c0->sm_count, st));
@@ -2526,10 +2541,7 @@ int ps2_shard_bin(ps2_ctx* c, void* d_grid) {
     t.ph_res = c->ph_res.p;
     CK(launch_snr_weight(t, c->amp.as<float>(), c->w.p, fp64, c->sm_count, c->st));
   }
-  CK(cudaMemsetAsync(c->hist.p, 0, sizeof(int32_t) * PS2_COH_BINS, c->st));
-  CK(cudaMemsetAsync(c->n_invalid.p, 0, sizeof(int32_t), c->st));
-  CK(cudaMemsetAsync(c->rms_partial.p, 0, sizeof(double) * c->topo_blocks, c->st));
-  if (later && c->psquare) CK(launch_psquare_weights(bin_args(c, 1, c->K[0].p), c->N, fp64, c->sm_count, c->st));
+  CK(launch_iter_begin(begin_args(c, later), fp64, c->sm_count, c->st));
   CK(launch_bin(bin_args(c, 0, c->K[0].p), fp64, c->sm_count, c->st));
   CK(cudaMemcpyAsync(d_grid, c->grid.p, csz(c) * c->G * c->Mp, cudaMemcpyDeviceToDevice, c->st));
   CK(cudaStreamSynchronize(c->st));
@@ -2588,7 +2600,6 @@ int ps2_shard_fit(ps2_ctx* c, double* stats) {
   if (!c || !c->loaded) return set_err(PS2_ERR_NOT_LOADED, "ps2_shard_fit: no patch loaded");
   if (!stats) return set_err(PS2_ERR_INVALID_ARG, "ps2_shard_fit: NULL statistics");
   CK(cudaSetDevice(c->device));
-  CK(cudaMemcpyAsync(c->K[1].p, c->K[0].p, rsz(c) * c->N, cudaMemcpyDeviceToDevice, c->st));
   TopoArgs t = topo_args(c, c->K[0].p, c->C.p, c->coh.p);
   if (!c->psquare) t.ph_res = c->ph_res.p;
   CK(launch_topofit(t, c->fp64, c->topo_blocks, c->st));

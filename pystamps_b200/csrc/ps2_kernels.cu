@@ -100,13 +100,10 @@ __device__ __forceinline__ float2 mk(float a, float b) { return make_float2(a, b
 __device__ __forceinline__ double2 mk(double a, double b) { return make_double2(a, b); }
 
 // ============================================================= binning ====
-template <typename R, int MODE>
-__device__ __forceinline__ R bin_weight(const BinArgs& a, const R* __restrict__ W, const R* __restrict__ coh,
-                                        const int s) {
-  if (MODE == 3) return R(1);
-  if (MODE != 1) return W[s];
-  // psquare_weighting lookup (native_stage2.rs:1674-1682)
-  const double v = __dmul_rn(static_cast<double>(coh[s]), 1000.0);
+// psquare_weighting lookup (native_stage2.rs:1674-1682)
+template <typename R>
+__device__ __forceinline__ R psquare_weight(const BinArgs& a, const R coh) {
+  const double v = __dmul_rn(static_cast<double>(coh), 1000.0);
   double r = v >= 0.0 ? floor(__dadd_rn(v, 0.5)) : ceil(__dsub_rn(v, 0.5));
   r = fmin(fmax(r, 0.0), static_cast<double>(a.lut_len - 1));
   const int ix = isnan(r) ? 0 : static_cast<int>(r);
@@ -121,8 +118,7 @@ __device__ __forceinline__ void bin_task_t(const BinArgs& a, const int64_t task,
   using C = typename CT<R>::C;
   const float2* __restrict__ ph = static_cast<const float2*>(a.ph_nm);
   const R* __restrict__ K = static_cast<const R*>(a.K);
-  R* __restrict__ W = static_cast<R*>(a.w);
-  const R* __restrict__ coh = static_cast<const R*>(a.coh);
+  const R* __restrict__ W = static_cast<const R*>(a.w);
   C* __restrict__ grid = static_cast<C*>(a.grid);
   const float* __restrict__ bp = a.bp;
   const int64_t M = a.M;
@@ -131,7 +127,6 @@ __device__ __forceinline__ void bin_task_t(const BinArgs& a, const int64_t task,
     const int chunk = static_cast<int>(task - cell * a.nchunk);
     const int c = chunk * 32 + lane;
     const bool active = c < a.M;
-    const bool write_w = MODE == 1 && chunk == 0 && lane == 0;
     const int s0 = a.cell_start[cell], s1 = a.cell_start[cell + 1];
     R ax = R(0), ay = R(0);
     // rows are taken eight at a time with every load issued before the
@@ -147,7 +142,7 @@ __device__ __forceinline__ void bin_task_t(const BinArgs& a, const int64_t task,
         bv[i] = R(0);
         v[i] = make_float2(0.f, 0.f);
         if (s < s1) {
-          wv[i] = bin_weight<R, MODE>(a, W, coh, s);
+          wv[i] = MODE == 3 ? R(1) : W[s];
           if (MODE != 3) kv[i] = K[s];
           if (active) {
             v[i] = ph[static_cast<int64_t>(s) * M + c];
@@ -160,7 +155,6 @@ __device__ __forceinline__ void bin_task_t(const BinArgs& a, const int64_t task,
       for (int i = 0; i < 8; ++i) {
         const int s = sb + i;
         if (s >= s1) break;
-        if (write_w) W[s] = wv[i];
         if (!active) continue;
         if (MODE == 3) {
           // accumulate_grid alone: ph_nm holds ph_weight, no ramp and no weight
@@ -180,27 +174,38 @@ __device__ __forceinline__ void bin_task_t(const BinArgs& a, const int64_t task,
   }
 }
 
-// The P-square weights of every row from its previous coherence and the table
-// of the last update (psquare_weighting's lookup, native_stage2.rs:1674-1682),
-// the same function bin_weight applies in mode 1, as one elementwise pass ahead
-// of binning: the binning warps then read w (mode 0) instead of each lane of
-// each interferogram chunk repeating the lookup and its dependent table load.
+// What an iteration needs before its binning, as one elementwise pass: K[1] <-
+// K[0] (the K this iteration bins with; topofit rewrites K[0] in place), the
+// statistics cleared and, from the second iteration on with P-square weighting,
+// the weights of every row from its previous coherence and the table of the
+// last update (the lookup once per row, not by each lane of each interferogram
+// chunk inside the binning). One launch in the place of three memsets, a copy
+// and a weights kernel: an iteration of a 20,000 PS x 20 patch is launch-bound
+// (11 nodes -> 6 with the loop condition set by k_finalize).
 template <typename R>
-__global__ void __launch_bounds__(256) k_psquare_weights(BinArgs a, int64_t N) {
-  const R* __restrict__ coh = static_cast<const R*>(a.coh);
-  R* __restrict__ W = static_cast<R*>(a.w);
+__global__ void __launch_bounds__(256) k_iter_begin(BeginArgs a) {
+  const R* __restrict__ K0 = static_cast<const R*>(a.bin.K);
+  R* __restrict__ K1 = static_cast<R*>(a.K1);
+  R* __restrict__ W = static_cast<R*>(a.bin.w);
+  const R* __restrict__ coh = static_cast<const R*>(a.bin.coh);
+  const int64_t t0 = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
   const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
-  for (int64_t s = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s < N; s += stride)
-    W[s] = bin_weight<R, 1>(a, W, coh, static_cast<int>(s));
+  for (int64_t i = t0; i < a.n_partial; i += stride) a.rms_partial[i] = 0.0;
+  if (t0 < kCohBins) a.hist[t0] = 0;
+  if (t0 == 0) *a.n_invalid = 0;
+  for (int64_t s = t0; s < a.N; s += stride) {
+    K1[s] = K0[s];
+    if (a.weights) W[s] = psquare_weight<R>(a.bin, coh[s]);
+  }
 }
 
-cudaError_t launch_psquare_weights(const BinArgs& a, int64_t N, bool fp64, int sm_count, cudaStream_t st) {
-  if (N <= 0) return cudaSuccess;
-  const int64_t blocks = std::min<int64_t>((N + 255) / 256, static_cast<int64_t>(sm_count) * 16);
+cudaError_t launch_iter_begin(const BeginArgs& a, bool fp64, int sm_count, cudaStream_t st) {
+  const int64_t blocks =
+      std::max<int64_t>(1, std::min<int64_t>((a.N + 255) / 256, static_cast<int64_t>(sm_count) * 16));
   if (fp64)
-    k_psquare_weights<double><<<static_cast<unsigned>(blocks), 256, 0, st>>>(a, N);
+    k_iter_begin<double><<<static_cast<unsigned>(blocks), 256, 0, st>>>(a);
   else
-    k_psquare_weights<float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(a, N);
+    k_iter_begin<float><<<static_cast<unsigned>(blocks), 256, 0, st>>>(a);
   return cudaGetLastError();
 }
 
@@ -210,8 +215,6 @@ template <typename R>
 __device__ __forceinline__ void bin_task(const BinArgs& a, const int64_t task, const int lane) {
   if (a.mode == 3)
     bin_task_t<R, 3, false>(a, task, lane);
-  else if (a.mode == 1)
-    a.bp_row_inv ? bin_task_t<R, 1, true>(a, task, lane) : bin_task_t<R, 1, false>(a, task, lane);
   else
     a.bp_row_inv ? bin_task_t<R, 0, true>(a, task, lane) : bin_task_t<R, 0, false>(a, task, lane);
 }
@@ -2198,16 +2201,39 @@ cudaError_t launch_topofit(const TopoArgs& a, bool fp64, int grid_blocks, cudaSt
 // P-square update (:364-381, :1642-1683) producing the prand_hi table that the
 // next k_bin turns into weights. Sums use explicit _rn arithmetic and the
 // reference's order so the table matches the reference given equal inputs.
+//
+// One block, bound by the latency of its serial parts: the operands are fetched
+// together up front, the two ordered sums run in two warps at once, and an
+// interpolated value adds only the 8 taps that meet a sample (the other 71
+// multiply a zero). 33 -> 4.4 us a launch.
 __device__ __forceinline__ void finalize_body(const FinalizeArgs& a) {
   __shared__ double sh[256];
-  __shared__ double na[kCohBins], prand[kCohBins], interp_in[kCohBins + 1];
-  __shared__ double scale_s;
+  __shared__ double na[kCohBins], nr[kCohBins], prand[kCohBins], interp_in[kCohBins + 1], taps[80];
+  __shared__ double num_s, den_s;
   __shared__ int go_on;
   const int tid = threadIdx.x;
+  double st0 = 0.0, st1 = 0.0;
+  int inv = 0;
+  if (tid == 0) {
+    st0 = a.state[0];
+    st1 = a.state[1];
+    inv = *a.n_invalid;
+  }
+  if (tid < kCohBins) {
+    na[tid] = static_cast<double>(a.hist[tid]);
+    nr[tid] = a.nr_scaled[tid];
+  }
+  if (tid >= 128 && tid < 128 + 79) taps[tid - 128] = a.taps79[tid - 128];
   double s = 0.0;
-  for (int i = tid; i < a.n_partial; i += 256) s += a.rms_partial[i];
+  for (int i0 = tid; i0 < a.n_partial; i0 += 256 * 10) {
+    double v[10];
+#pragma unroll
+    for (int u = 0; u < 10; ++u) v[u] = i0 + 256 * u < a.n_partial ? a.rms_partial[i0 + 256 * u] : 0.0;
+#pragma unroll
+    for (int u = 0; u < 10; ++u)
+      if (i0 + 256 * u < a.n_partial) s += v[u];
+  }
   sh[tid] = s;
-  if (tid < kCohBins) na[tid] = static_cast<double>(a.hist[tid]);
   __syncthreads();
   for (int w = 128; w > 0; w >>= 1) {
     if (tid < w) sh[tid] += sh[tid + w];
@@ -2215,9 +2241,9 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a) {
   }
   if (tid == 0) {
     const double rms = sqrt(sh[0] / static_cast<double>(a.N > 0 ? a.N : 1));
-    const double gcs = a.state[0];
+    const double gcs = st0;
     const double delta = rms - gcs;
-    const int64_t i_loop = static_cast<int64_t>(a.state[1]);
+    const int64_t i_loop = static_cast<int64_t>(st1);
     const int64_t cap = a.gamma_max_iterations > 1 ? a.gamma_max_iterations : 1;
     const bool stop = fabs(delta) < a.gamma_change_convergence || i_loop >= cap;
     a.state[0] = rms;
@@ -2228,26 +2254,23 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a) {
     a.stats_out[1] = rms;
     a.stats_out[2] = delta;
     a.stats_out[3] = stop ? 1.0 : 0.0;
-    a.stats_out[4] = static_cast<double>(*a.n_invalid);
+    a.stats_out[4] = static_cast<double>(inv);
     go_on = ((!stop || a.force_continue) && a.psquare) ? 1 : 0;
-    if (go_on) {
-      // Nr rescaled so its low-coherence mass matches Na's (sequential sums)
-      double den = 0.0;
-      for (int i = 0; i < a.low_coh_thresh; ++i) den = __dadd_rn(den, a.nr_scaled[i]);
-      double sc = 1.0;
-      if (den > 0.0) {
-        double num = 0.0;
-        for (int i = 0; i < a.low_coh_thresh; ++i) num = __dadd_rn(num, na[i]);
-        sc = num / den;
-      }
-      scale_s = sc;
-      interp_in[0] = 1.0;
-    }
+    interp_in[0] = 1.0;
+  } else if (tid == 32) {
+    // Nr rescaled so its low-coherence mass matches Na's (sequential sums)
+    double den = 0.0;
+    for (int i = 0; i < a.low_coh_thresh; ++i) den = __dadd_rn(den, nr[i]);
+    den_s = den;
+  } else if (tid == 64) {
+    double num = 0.0;
+    for (int i = 0; i < a.low_coh_thresh; ++i) num = __dadd_rn(num, na[i]);
+    num_s = num;
   }
   __syncthreads();
   if (!go_on) return;
   if (tid < kCohBins) {
-    const double nrv = __dmul_rn(a.nr_scaled[tid], scale_s);
+    const double nrv = __dmul_rn(nr[tid], den_s > 0.0 ? num_s / den_s : 1.0);
     a.nr_scaled[tid] = nrv;
     const double d = na[tid] == 0.0 ? 1.0 : na[tid];
     double p = fmin(nrv / d, 1.0);
@@ -2260,6 +2283,7 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a) {
   if (tid < kCohBins) {
     const int ix = tid + 7;
     double acc = 0.0;
+#pragma unroll
     for (int k = 0; k < 7; ++k) {
       const int j = ix - k;
       const double v = j < 7 ? 1.0 : prand[j - 7];
@@ -2268,31 +2292,25 @@ __device__ __forceinline__ void finalize_body(const FinalizeArgs& a) {
     interp_in[1 + tid] = acc / a.g7sum;
   }
   __syncthreads();
-  // matlab_interp(.., 10) with the 79-tap FIR, delay 39, tail trimmed to 1001
+  // matlab_interp(.., 10) with the 79-tap FIR, delay 39, tail trimmed to 1001:
+  // tap k meets sample (n - k) / 10 where that is whole, in tap order
   for (int i = tid; i < 1001; i += 256) {
     const int n = i + 39;
     double acc = 0.0;
-    for (int k = 0; k < 79; ++k) {
-      const int p = n - k;
-      if (p < 0) continue;
-      const double v = (p % 10 == 0 && p / 10 < 101) ? interp_in[p / 10] : 0.0;
-      acc = __dadd_rn(acc, __dmul_rn(a.taps79[k], v));
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const int k = n % 10 + 10 * j, q = n / 10 - j;
+      if (k < 79 && q >= 0 && q < 101) acc = __dadd_rn(acc, __dmul_rn(taps[k], interp_in[q]));
     }
     a.lut[i] = __dmul_rn(acc, 10.0);
   }
 }
 
-__global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) { finalize_body(a); }
-
-// Body tail of the graph that runs the loop to convergence: keep looping while
-// the finalize of this iteration did not raise the stop flag.
-__global__ void k_loop_continue(cudaGraphConditionalHandle h, const double* stats) {
-  if (threadIdx.x == 0) cudaGraphSetConditional(h, stats[3] == 0.0 ? 1u : 0u);
-}
-
-cudaError_t launch_loop_continue(cudaGraphConditionalHandle h, const double* stats, cudaStream_t st) {
-  k_loop_continue<<<1, 32, 0, st>>>(h, stats);
-  return cudaGetLastError();
+// In the graph that runs the loop to convergence this is the body's last node:
+// it keeps the loop going while it has not raised the stop flag.
+__global__ void __launch_bounds__(256) k_finalize(FinalizeArgs a) {
+  finalize_body(a);
+  if (a.set_loop && threadIdx.x == 0) cudaGraphSetConditional(a.loop, a.stats_out[3] == 0.0 ? 1u : 0u);
 }
 
 cudaError_t launch_finalize(const FinalizeArgs& a, cudaStream_t st) {
@@ -3112,18 +3130,30 @@ __device__ __forceinline__ int find_patch(const int64_t* __restrict__ prefix, in
   return lo;
 }
 
-// per-iteration reset of the active patches: histogram, invalid count, rms
-// partials, and K[1] <- K[0] (the K this iteration bins with)
-__global__ void __launch_bounds__(256) k_batch_reset(BatchArgs b) {
-  const int p = blockIdx.x;
-  if (p >= b.P || !b.active[p]) return;
-  const PatchDev& d = b.patch[p];
-  for (int i = threadIdx.x; i < kCohBins; i += blockDim.x) d.topo.hist[i] = 0;
-  if (threadIdx.x == 0) *d.topo.n_invalid = 0;
-  for (int i = threadIdx.x; i < d.fin.n_partial; i += blockDim.x) d.topo.rms_partial[i] = 0.0;
-  const float* __restrict__ k0 = static_cast<const float*>(d.bin.K);
-  float* __restrict__ k1 = d.K1;
-  for (int64_t i = threadIdx.x; i < d.topo.N; i += blockDim.x) k1[i] = k0[i];
+// k_iter_begin over the active patches: their statistics cleared (a block per
+// patch), K[1] <- K[0] and the P-square weights from iteration 2 on (elements
+// numbered patch after patch over the whole grid). A block per patch copying its
+// K took 0.22 ms an iteration of 12 patches of up to 200,000 PS, and the weights
+// were looked up by every lane of every interferogram chunk of the binning.
+__global__ void __launch_bounds__(256) k_batch_begin(BatchArgs b) {
+  for (int p = blockIdx.x; p < b.P; p += gridDim.x) {
+    if (!b.active[p]) continue;
+    const PatchDev& d = b.patch[p];
+    for (int i = threadIdx.x; i < kCohBins; i += blockDim.x) d.topo.hist[i] = 0;
+    if (threadIdx.x == 0) *d.topo.n_invalid = 0;
+    for (int i = threadIdx.x; i < d.fin.n_partial; i += blockDim.x) d.topo.rms_partial[i] = 0.0;
+  }
+  const int64_t total = b.ps_prefix[b.P];
+  for (int64_t u = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; u < total;
+       u += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int p = find_patch(b.ps_prefix, b.P, u);
+    if (!b.active[p]) continue;
+    const PatchDev& d = b.patch[p];
+    const int64_t s = u - b.ps_prefix[p];
+    d.K1[s] = static_cast<const float*>(d.bin.K)[s];
+    if (d.psquare && d.fin.state[1] > 1.0)
+      static_cast<float*>(d.bin.w)[s] = psquare_weight<float>(d.bin, static_cast<const float*>(d.bin.coh)[s]);
+  }
 }
 
 __global__ void __launch_bounds__(256) k_batch_bin(BatchArgs b) {
@@ -3134,11 +3164,7 @@ __global__ void __launch_bounds__(256) k_batch_bin(BatchArgs b) {
   for (int64_t u = gw; u < total; u += nw) {
     const int p = find_patch(b.bin_prefix, b.P, u);
     if (!b.active[p]) continue;
-    const PatchDev& d = b.patch[p];
-    BinArgs a = d.bin;
-    // iteration 1 bins with the initial weights, later ones with the P-square table
-    a.mode = (d.psquare && d.fin.state[1] > 1.0) ? 1 : 0;
-    bin_task<float>(a, u - b.bin_prefix[p], lane);
+    bin_task<float>(b.patch[p].bin, u - b.bin_prefix[p], lane);
   }
 }
 
@@ -3213,8 +3239,10 @@ __global__ void k_batch_continue(cudaGraphConditionalHandle h, const int* n_acti
   if (threadIdx.x == 0) cudaGraphSetConditional(h, *n_active > 0 ? 1u : 0u);
 }
 
-cudaError_t launch_batch_reset(const BatchArgs& b, cudaStream_t st) {
-  k_batch_reset<<<b.P, 256, 0, st>>>(b);
+cudaError_t launch_batch_begin(const BatchArgs& b, int64_t total_ps, int sm_count, cudaStream_t st) {
+  const int64_t blocks =
+      std::max<int64_t>(1, std::min<int64_t>((total_ps + 255) / 256, static_cast<int64_t>(sm_count) * 8));
+  k_batch_begin<<<static_cast<unsigned>(blocks), 256, 0, st>>>(b);
   return cudaGetLastError();
 }
 

@@ -26,13 +26,25 @@ struct BinArgs {
   int64_t G;
   int M, Mp, nchunk;
   const void* K;         // real [N] (sorted)
-  void* w;               // real [N] (sorted): read (mode 0) or written (mode 1)
-  const void* coh;       // real [N] previous coherence (mode 1)
-  const double* lut;     // P-square prand_hi table (mode 1)
+  void* w;               // real [N] (sorted); written by k_iter_begin
+  const void* coh;       // real [N] previous coherence (k_iter_begin)
+  const double* lut;     // P-square prand_hi table (k_iter_begin)
   int lut_len;
-  int mode;              // 0: w given; 1: w = (1 - lut[round(1000 coh)])^2
+  int mode;              // 0: phase ramp and weights w; 3: ph_nm holds ph_weight (plain sum)
   void* grid;            // complex [G, Mp]
   int blocks_per_sm;     // launch shape: resident blocks per SM (0: as many as fit)
+};
+
+// ---------------------------------------------------- start of an iteration --
+struct BeginArgs {
+  BinArgs bin;          // K (= K[0]), w, coh and lut
+  void* K1;             // real [N]: the K this iteration bins with
+  int64_t N;
+  int weights;          // 1: w = (1 - lut[round(1000 coh)])^2
+  int32_t* hist;        // cleared: [100]
+  int32_t* n_invalid;   // cleared: [1]
+  double* rms_partial;  // cleared: [n_partial]
+  int n_partial;
 };
 
 // ------------------------------------------------------------------ CLAP --
@@ -111,6 +123,8 @@ struct FinalizeArgs {
   double* stats_out;         // [6] per-iteration record
   int32_t* n_invalid;
   int force_continue;        // iterate past the stop rule (timing runs)
+  int set_loop;              // 1: last node of a WHILE body, sets its condition
+  cudaGraphConditionalHandle loop;
 };
 
 // --------------------------------------------------------------- stage 3 --
@@ -149,7 +163,7 @@ struct S3FitArgs {
 // --------------------------------------------------------------- batches --
 // One patch of a batch: the single-patch arguments of every step.
 struct PatchDev {
-  BinArgs bin;        // bin.K = K[0]; mode is set per iteration from fin.state
+  BinArgs bin;        // bin.K = K[0]
   ClapArgs clap;
   OverlapArgs ov;
   TopoArgs topo;
@@ -168,6 +182,7 @@ struct BatchArgs {
   const int64_t* bin_prefix;  // [P + 1] warp-tasks (G * nchunk)
   const int64_t* clap_prefix; // [P + 1] block-tasks (W * Mp / 4)
   const int64_t* ov_prefix;   // [P + 1] elements (G * Mp)
+  const int64_t* ps_prefix;   // [P + 1] PS
 };
 
 // -------------------------------------------------------------- adjoints --
@@ -199,8 +214,7 @@ struct ClapBwdArgs {
 
 // ---------------------------------------------------------- launchers -----
 cudaError_t launch_bin(const BinArgs& a, bool fp64, int sm_count, cudaStream_t st);
-// w[s] = (1 - lut[round(1000 coh[s])])^2 for s < N (a.coh, a.lut, a.lut_len, a.w)
-cudaError_t launch_psquare_weights(const BinArgs& a, int64_t N, bool fp64, int sm_count, cudaStream_t st);
+cudaError_t launch_iter_begin(const BeginArgs& a, bool fp64, int sm_count, cudaStream_t st);
 cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32f& tf, const Twiddles32d& td, int sm_count,
                         cudaStream_t st);
 cudaError_t launch_overlap(const OverlapArgs& a, bool fp64, cudaStream_t st);
@@ -208,7 +222,6 @@ cudaError_t launch_topofit(const TopoArgs& a, bool fp64, int grid_blocks, cudaSt
 int topofit_grid_blocks(int sm_count, bool fp64);
 int topofit_lanes(int M);
 cudaError_t launch_finalize(const FinalizeArgs& a, cudaStream_t st);
-cudaError_t launch_loop_continue(cudaGraphConditionalHandle h, const double* stats, cudaStream_t st);
 cudaError_t launch_coh(const CohArgs& a, int which /*0 fwd, 1 coherence bwd, 2 bin bwd*/, bool fp64,
                        int sm_count, cudaStream_t st);
 cudaError_t launch_cell_sum(const CohArgs& a, const int32_t* cell_start, int64_t G, void* out, bool fp64,
@@ -229,7 +242,7 @@ int64_t clap_part_elems(int nwi, int nwj, int n_win, int Mp);
 // window blocks per axis (4 windows a side) of the fused CLAP
 int clap_block_count(int nw_axis);
 cudaError_t topofit_geometry(const TopoArgs& a, int grid_cap, int* L_out, int* mpad_out, int* blocks_out);
-cudaError_t launch_batch_reset(const BatchArgs& b, cudaStream_t st);
+cudaError_t launch_batch_begin(const BatchArgs& b, int64_t total_ps, int sm_count, cudaStream_t st);
 cudaError_t launch_s3_clap(const S3ClapArgs& a, const Twiddles32f& tf, int sm_count, cudaStream_t st);
 cudaError_t launch_s3_fit(const S3FitArgs& a, int sm_count, cudaStream_t st);
 
