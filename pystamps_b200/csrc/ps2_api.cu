@@ -111,8 +111,7 @@ class DeviceCache {
         *p = l[best].first;
         *bytes = l[best].second;
         held_[dev] -= *bytes;
-        l[best] = l.back();
-        l.pop_back();
+        l.erase(l.begin() + static_cast<std::ptrdiff_t>(best));
         return cudaSuccess;
       }
     }
@@ -129,12 +128,21 @@ class DeviceCache {
     int dev = 0;
     if (g_call_stream && bytes <= kMaxBlock && cudaGetDevice(&dev) == cudaSuccess && dev == device &&
         dev < kMaxDevices && cudaStreamSynchronize(g_call_stream) == cudaSuccess) {
-      std::lock_guard<std::mutex> g(mu_);
-      if (held_[dev] + bytes <= kMaxBytes) {
-        blocks_[dev].emplace_back(p, bytes);
+      std::vector<void*> old;  // the longest-kept blocks make room
+      {
+        std::lock_guard<std::mutex> g(mu_);
+        auto& l = blocks_[dev];
+        size_t k = 0;
+        for (; k < l.size() && held_[dev] + bytes > kMaxBytes; ++k) {
+          held_[dev] -= l[k].second;
+          old.push_back(l[k].first);
+        }
+        l.erase(l.begin(), l.begin() + static_cast<std::ptrdiff_t>(k));
+        l.emplace_back(p, bytes);
         held_[dev] += bytes;
-        return;
       }
+      for (void* q : old) cudaFree(q);
+      return;
     }
     cudaFree(p);
   }
