@@ -1,0 +1,378 @@
+// The FP32 CLAP kernels (clap_f32.cuh): one patch's windows and a batch's.
+#include <algorithm>
+
+#include "clap_f32.cuh"
+
+namespace ps2 {
+
+cudaError_t kernel_attributes_once(size_t dynamic_smem);
+
+namespace {
+
+// Row stride of the pyramid-weight table: lane l reads row l, so rows 33 words
+// apart put the lanes on different banks.
+constexpr int kWtStride = 33;
+
+template <int NW>
+struct ClapSmemF {
+  ClapTileF<NW == 8 ? 4 : 8> tiles[NW];
+  float lp[1024];
+  float wt[32 * kWtStride];
+};
+
+template <int NW>
+__device__ __forceinline__ void clap_consts_f(const ClapArgs& a, ClapSmemF<NW>& m) {
+  const int nw2 = a.n_win * a.n_win;
+  for (int i = threadIdx.x; i < 1024; i += 32 * NW) m.lp[i] = static_cast<float>(a.low_pass[i]);
+  for (int i = threadIdx.x; i < nw2; i += 32 * NW)
+    m.wt[(i / a.n_win) * kWtStride + i % a.n_win] = static_cast<float>(a.wscaled[i]);
+}
+
+// One window in its tile: on entry the window zero-padded to 32 x 32 (NWIN = 0; a
+// compile-time window's padding is never stored), on exit rows and columns < n_win
+// hold the filtered values times the pyramid weight / 1024, real parts in im and
+// imaginary parts in re.
+template <int NWIN, typename Tile>
+__device__ __forceinline__ void window_f(Tile& T, const int lane, const ClapArgs& a, const float* lp, const float* wt,
+                                         const float (&g)[4], const int rs, const int cs) {
+  constexpr int NZ = NWIN > 0 ? NWIN : 32;
+  const int nw = NWIN > 0 ? NWIN : a.n_win;
+  const float* wrow = wt + (lane - rs) * kWtStride - cs;
+#pragma unroll 1
+  for (int half = 0; half < 2; ++half) {
+#pragma unroll 1
+    for (int p = 2 * half; p < 2 * half + 2; ++p) fft_row<NZ>(T, lane, p, wrow, rs, cs, nw);
+    if (half == 0) {
+      float o[32];
+      smooth_tile(T, lane, g, o);
+      float v0, v1;
+      median_pair1024(o, &T.hs[0][0], v0, v1);
+      gain_tile(T, lane, o, (v0 + v1) * 0.5f, a.alpha_is_one, static_cast<float>(a.alpha), static_cast<float>(a.beta),
+                lp);
+    }
+  }
+}
+
+constexpr int kLoadU = 9;  // 16-byte accesses in flight per thread of the window loads
+
+// Window (ix1, ix2) of interferograms NW g .. NW g + NW - 1 through the block's
+// tiles: clap_windows' corner (native_stage2.rs:957-995) returned in i1, j1; on
+// exit the tiles hold the weighted filtered window.
+template <int NW, int NWIN>
+__device__ __forceinline__ void compute_f(const ClapArgs& a, const int ix1, const int ix2, const int g,
+                                          ClapSmemF<NW>& m, const float (&g7)[4], int& i1, int& j1) {
+  constexpr int NT = 32 * NW, NQ = NW / 2;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int nw = NWIN > 0 ? NWIN : a.n_win, nw2 = nw * nw;
+  const int n_inc = nw / 4 > 1 ? nw / 4 : 1;
+  const float2* __restrict__ grid = static_cast<const float2*>(a.grid);
+  i1 = ix1 * n_inc;
+  int rs = 0;
+  if (i1 + nw > a.n_i) {
+    rs = i1 + nw - a.n_i;
+    i1 = a.n_i - nw;
+  }
+  j1 = ix2 * n_inc;
+  int cs = 0;
+  if (j1 + nw > a.n_j) {
+    cs = j1 + nw - a.n_j;
+    j1 = a.n_j - nw;
+  }
+  __syncthreads();
+  if (NWIN == 0 && nw < 32) {
+    for (int idx = tid; idx < NW * 1024; idx += NT) {
+      const int q = idx >> 10, r = (idx >> 5) & 31, c = idx & 31;
+      if (r >= nw || c >= nw) m.tiles[q].re[r][c] = m.tiles[q].im[r][c] = 0.f;
+    }
+  }
+  // pixel -> (row, column) by pix * inv_nw >> 16, exact for pix < 1024 and nw <= 32
+  const uint32_t inv_nw = (65536u + static_cast<uint32_t>(nw) - 1u) / static_cast<uint32_t>(nw);
+  // a thread's pixels are NT / NQ apart: row and column step by step, with one carry
+  const int q = (tid % NQ) * 2, c = NW * g + q, pix0 = tid / NQ;
+  const int dli = (NT / NQ) / nw, dlj = (NT / NQ) - dli * nw;
+  int li = static_cast<int>((static_cast<uint32_t>(pix0) * inv_nw) >> 16), lj = pix0 - li * nw;
+  // columns M .. Mp - 1 of the grid are zero, c is even and Mp a multiple of 4
+  const float2* src = grid + (static_cast<int64_t>(i1 + li) * a.n_j + (j1 + lj)) * a.Mp + c;
+  const int64_t step = (static_cast<int64_t>(dli) * a.n_j + dlj) * a.Mp;
+  const int64_t carry = static_cast<int64_t>(a.n_j - nw) * a.Mp;
+  const int pix_end = c < a.Mp ? nw2 : 0;
+  float* re0 = &m.tiles[q].re[0][0];
+  constexpr int kIm = 32 * kTileRow, kNext = sizeof(m.tiles[0]) / sizeof(float);  // tile q's im, tile q + 1
+  for (int p0 = pix0; p0 < nw2; p0 += (NT / NQ) * kLoadU) {
+    float4 v[kLoadU];
+    int at[kLoadU];
+#pragma unroll
+    for (int u = 0; u < kLoadU; ++u) {
+      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      at[u] = li * kTileRow + lj;
+      if (p0 + u * (NT / NQ) < pix_end) v[u] = *reinterpret_cast<const float4*>(src);
+      src += step;
+      li += dli;
+      lj += dlj;
+      if (lj >= nw) {
+        lj -= nw;
+        ++li;
+        src += carry;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < kLoadU; ++u) {
+      if (p0 + u * (NT / NQ) < nw2) {
+        float4 x = v[u];
+        if (isnan(x.x) || isnan(x.y)) x.x = x.y = 0.f;  // NaN -> 0 (clap_filter_one_ifg)
+        if (isnan(x.z) || isnan(x.w)) x.z = x.w = 0.f;
+        re0[at[u]] = x.x;
+        re0[at[u] + kIm] = x.y;
+        re0[at[u] + kNext] = x.z;
+        re0[at[u] + kNext + kIm] = x.w;
+      }
+    }
+  }
+  __syncthreads();
+  if (NW * g + warp < a.M) {
+    window_f<NWIN>(m.tiles[warp], lane, a, m.lp, m.wt, g7, rs, cs);
+  } else {
+    // an interferogram of the padding: zeros for the window stack
+    for (int i = lane; i < nw * nw; i += 32) m.tiles[warp].re[i / nw][i % nw] = m.tiles[warp].im[i / nw][i % nw] = 0.f;
+  }
+  __syncthreads();
+}
+
+template <int NW>
+__host__ __device__ __forceinline__ int groups_f(const int Mp) {
+  return (Mp + NW - 1) / NW;
+}
+
+// One block-task of the window-stack form: window a.w_lo + task / groups.
+template <int NW, int NWIN>
+__device__ __forceinline__ void task_f(const ClapArgs& a, const int64_t task, ClapSmemF<NW>& m, const float (&g7)[4]) {
+  constexpr int NT = 32 * NW, NQ = NW / 2;
+  const int groups = groups_f<NW>(a.Mp);
+  const int nw = NWIN > 0 ? NWIN : a.n_win, nw2 = nw * nw;
+  // windows number nwi * nwj < 2^31 / 36 cells: 32-bit divisions
+  const int w = static_cast<int>(task < INT32_MAX ? static_cast<uint32_t>(task) / static_cast<uint32_t>(groups)
+                                                  : task / groups);
+  const int g = static_cast<int>(task - static_cast<int64_t>(w) * groups);
+  const int64_t wi = a.w_lo + w;
+  const int ix1 = static_cast<int>(static_cast<uint32_t>(wi) / static_cast<uint32_t>(a.nwj));
+  const int ix2 = static_cast<int>(wi) - ix1 * a.nwj;
+  int i1, j1;
+  compute_f<NW, NWIN>(a, ix1, ix2, g, m, g7, i1, j1);
+  const uint32_t inv_nw = (65536u + static_cast<uint32_t>(nw) - 1u) / static_cast<uint32_t>(nw);
+  float2* out = static_cast<float2*>(a.win_out);
+  const int q = (threadIdx.x % NQ) * 2, c = NW * g + q, pix0 = threadIdx.x / NQ;
+  if (c >= a.Mp) return;
+  const int dli = (NT / NQ) / nw, dlj = (NT / NQ) - dli * nw;
+  int li = static_cast<int>((static_cast<uint32_t>(pix0) * inv_nw) >> 16), lj = pix0 - li * nw;
+  constexpr int kIm = 32 * kTileRow, kNext = sizeof(m.tiles[0]) / sizeof(float);
+  const float* re0 = &m.tiles[q].re[0][0];
+  float2* dst = out + (wi * nw2 + pix0) * a.Mp + c;
+#pragma unroll 3
+  for (int pix = pix0; pix < nw2; pix += NT / NQ) {
+    const float* s = re0 + li * kTileRow + lj;
+    // Mp is a multiple of 4 and c even: c + 1 < Mp, 16-byte aligned
+    *reinterpret_cast<float4*>(dst) = make_float4(s[kIm], s[0], s[kNext + kIm], s[kNext]);
+    dst += static_cast<int64_t>(NT / NQ) * a.Mp;
+    li += dli;
+    lj += dlj;
+    if (lj >= nw) {
+      lj -= nw;
+      ++li;
+    }
+  }
+}
+
+// The weighted window added to (or, for a cell no earlier window of the block
+// covered, stored in) the block's partial sums: see clap_accum_tiles.
+constexpr int kAccU = 6;
+template <int NW>
+__device__ __forceinline__ void accum_f(const ClapArgs& a, const ClapSmemF<NW>& m, double2* __restrict__ part,
+                                           const int64_t blk, const int box, const int i1, const int j1, const int r0,
+                                           const int c0, const int pi1, const int pj1, const int g, const int nw,
+                                           const int nw2, const uint32_t inv_nw) {
+  constexpr int NT = 32 * NW, NI = NW;
+  const int n_items = nw2 * NI;
+  for (int b0 = threadIdx.x; b0 < n_items; b0 += NT * kAccU) {
+    double2 old[kAccU];
+    int64_t off[kAccU];
+    int li[kAccU], lj[kAccU], qq[kAccU];
+    bool live[kAccU], first[kAccU];
+#pragma unroll
+    for (int u = 0; u < kAccU; ++u) {
+      const int idx = b0 + u * NT;
+      const int pix = idx / NI, q = idx % NI, c = NI * g + q;
+      live[u] = idx < n_items && c < a.M;
+      li[u] = static_cast<int>((static_cast<uint32_t>(pix) * inv_nw) >> 16);
+      lj[u] = pix - li[u] * nw;
+      qq[u] = q;
+      const int ai = i1 + li[u], aj = j1 + lj[u];
+      first[u] = ai >= pi1 + nw && aj >= pj1 + nw;
+      off[u] = ((blk * box + (ai - r0)) * box + (aj - c0)) * a.Mp + c;
+      old[u] = make_double2(0.0, 0.0);
+      if (live[u] && !first[u]) old[u] = part[off[u]];
+    }
+#pragma unroll
+    for (int u = 0; u < kAccU; ++u) {
+      if (!live[u]) continue;
+      const double vx = static_cast<double>(m.tiles[qq[u]].im[li[u]][lj[u]]);
+      const double vy = static_cast<double>(m.tiles[qq[u]].re[li[u]][lj[u]]);
+      part[off[u]] = first[u] ? make_double2(vx, vy) : make_double2(__dadd_rn(old[u].x, vx), __dadd_rn(old[u].y, vy));
+    }
+  }
+}
+
+// One block-task of the fused form: window block a.w_lo + task / groups.
+template <int NW, int NWIN>
+__device__ __forceinline__ void block_task_f(const ClapArgs& a, const int64_t task, ClapSmemF<NW>& m,
+                                                const float (&g7)[4]) {
+  const int groups = groups_f<NW>(a.Mp);
+  const int nw = NWIN > 0 ? NWIN : a.n_win, nw2 = nw * nw;
+  const int n_inc = nw / 4 > 1 ? nw / 4 : 1;
+  const int box = clap_box(nw);
+  const int nbj = clap_block_rows(a.nwj);
+  const int64_t blk = a.w_lo + task / groups;
+  const int g = static_cast<int>(task - (blk - a.w_lo) * groups);
+  const int bi = static_cast<int>(blk / nbj), bj = static_cast<int>(blk - static_cast<int64_t>(bi) * nbj);
+  const int ixa = kClapBlockWin * bi, ixb = min(ixa + kClapBlockWin, a.nwi);
+  const int jxa = kClapBlockWin * bj, jxb = min(jxa + kClapBlockWin, a.nwj);
+  const int r0 = min(ixa * n_inc, a.n_i - nw), c0 = min(jxa * n_inc, a.n_j - nw);
+  const uint32_t inv_nw = (65536u + static_cast<uint32_t>(nw) - 1u) / static_cast<uint32_t>(nw);
+  constexpr int kNone = -(1 << 20);
+  for (int ix1 = ixa; ix1 < ixb; ++ix1) {
+    const int pi1 = ix1 > ixa ? min((ix1 - 1) * n_inc, a.n_i - nw) : kNone;
+    for (int ix2 = jxa; ix2 < jxb; ++ix2) {
+      const int pj1 = ix2 > jxa ? min((ix2 - 1) * n_inc, a.n_j - nw) : kNone;
+      int i1, j1;
+      compute_f<NW, NWIN>(a, ix1, ix2, g, m, g7, i1, j1);
+      accum_f<NW>(a, m, static_cast<double2*>(a.part), blk, box, i1, j1, r0, c0, pi1, pj1, g, nw, nw2, inv_nw);
+    }
+  }
+}
+
+__device__ __forceinline__ void taps_f(const ClapArgs& a, float (&g)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) g[i] = static_cast<float>(a.g7[i]);  // symmetric: taps 0..3
+}
+
+// FUSED: window blocks into the partials; otherwise windows into the window
+// stack. Sixteen warps an SM in two blocks of eight (shared memory and 128
+// registers allow no more). 256 x 256 cells x 150 ifg: 2.57 -> 1.85 ms a launch (4,850 instructions a
+// window and interferogram against 6,800).
+template <int NW, int NWIN, bool FUSED>
+__global__ void __launch_bounds__(32 * NW, NW == 8 ? 2 : 3) k_clap_f32(ClapArgs a) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ClapSmemF<NW>& m = *reinterpret_cast<ClapSmemF<NW>*>(smem_raw);
+  clap_consts_f<NW>(a, m);
+  float g7[4];
+  taps_f(a, g7);
+  const int64_t nunit = a.w_n > 0 ? a.w_n
+                        : FUSED ? static_cast<int64_t>(clap_block_rows(a.nwi)) * clap_block_rows(a.nwj)
+                                : static_cast<int64_t>(a.nwi) * a.nwj;
+  const int64_t ntask = nunit * groups_f<NW>(a.Mp);
+  for (int64_t task = blockIdx.x; task < ntask; task += gridDim.x) {
+    if constexpr (FUSED)
+      block_task_f<NW, NWIN>(a, task, m, g7);
+    else
+      task_f<NW, NWIN>(a, task, m, g7);
+  }
+}
+
+// Block-tasks numbered patch after patch; the per-patch constants are reloaded
+// where a block's tasks change patch. NWIN = 24 when every patch has that window.
+template <int NWIN>
+__global__ void __launch_bounds__(256, 2) k_batch_clap(BatchArgs b) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  ClapSmemF<8>& m = *reinterpret_cast<ClapSmemF<8>*>(smem_raw);
+  float g7[4];
+  int cur = -1;
+  const int64_t total = b.clap_prefix[b.P];
+  for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
+    const int p = find_patch(b.clap_prefix, b.P, u);
+    if (!b.active[p]) continue;
+    const ClapArgs& a = b.patch[p].clap;
+    if (p != cur) {
+      // the previous task's readers of lp / wt passed its last barrier
+      clap_consts_f<8>(a, m);
+      taps_f(a, g7);
+      cur = p;
+    }
+    if (a.part)
+      block_task_f<8, NWIN>(a, u - b.clap_prefix[p], m, g7);
+    else
+      task_f<8, NWIN>(a, u - b.clap_prefix[p], m, g7);
+  }
+}
+
+template <int NW, int NWIN, bool FUSED>
+cudaError_t launch_form(const ClapArgs& a, const int64_t ntask, int sm_count, cudaStream_t st) {
+  const size_t sm = sizeof(ClapSmemF<NW>);
+  cudaError_t e = kernel_attributes_once(sm);
+  if (e != cudaSuccess) return e;
+  int per_sm = 0;
+  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_clap_f32<NW, NWIN, FUSED>, 32 * NW, sm);
+  if (e != cudaSuccess) return e;
+  if (a.blocks_per_sm > 0 && a.blocks_per_sm < per_sm) per_sm = a.blocks_per_sm;
+  const int64_t blocks = std::min<int64_t>(ntask, static_cast<int64_t>(sm_count) * (per_sm > 0 ? per_sm : 1));
+  k_clap_f32<NW, NWIN, FUSED><<<static_cast<unsigned>(blocks), 32 * NW, sm, st>>>(a);
+  return cudaGetLastError();
+}
+
+template <int NW>
+cudaError_t launch_nw(const ClapArgs& a, int sm_count, cudaStream_t st) {
+  if (a.nwi <= 0 || a.nwj <= 0) return cudaSuccess;
+  const int64_t nunit = a.w_n > 0 ? a.w_n
+                        : a.part ? static_cast<int64_t>(clap_block_rows(a.nwi)) * clap_block_rows(a.nwj)
+                                 : static_cast<int64_t>(a.nwi) * a.nwj;
+  const int64_t ntask = nunit * groups_f<NW>(a.Mp);
+  if (ntask <= 0) return cudaSuccess;
+  if (a.n_win == 24)
+    return a.part ? launch_form<NW, 24, true>(a, ntask, sm_count, st)
+                  : launch_form<NW, 24, false>(a, ntask, sm_count, st);
+  return a.part ? launch_form<NW, 0, true>(a, ntask, sm_count, st)
+                : launch_form<NW, 0, false>(a, ntask, sm_count, st);
+}
+
+template <typename F>
+cudaError_t opt_in(F* f, int optin) {
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, f);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              optin - static_cast<int>(fa.sharedSizeBytes));
+}
+
+}  // namespace
+
+int64_t batch_clap_groups(int Mp) { return groups_f<8>(Mp); }
+
+cudaError_t launch_clap_f32(const ClapArgs& a, int sm_count, cudaStream_t st) {
+  return a.nw_block == 4 ? launch_nw<4>(a, sm_count, st) : launch_nw<8>(a, sm_count, st);
+}
+
+cudaError_t launch_batch_clap(const BatchArgs& b, int64_t total, bool win24, int sm_count, cudaStream_t st) {
+  if (total <= 0) return cudaSuccess;
+  const size_t sm = sizeof(ClapSmemF<8>);
+  cudaError_t e = kernel_attributes_once(sm);
+  if (e != cudaSuccess) return e;
+  const int64_t blocks = std::min<int64_t>(total, static_cast<int64_t>(sm_count) * 2);
+  if (win24)
+    k_batch_clap<24><<<static_cast<unsigned>(blocks), 256, sm, st>>>(b);
+  else
+    k_batch_clap<0><<<static_cast<unsigned>(blocks), 256, sm, st>>>(b);
+  return cudaGetLastError();
+}
+
+cudaError_t clap_f32_attributes(int optin) {
+  const cudaError_t steps[] = {
+      opt_in(k_clap_f32<4, 24, false>, optin), opt_in(k_clap_f32<4, 24, true>, optin),
+      opt_in(k_clap_f32<4, 0, false>, optin),  opt_in(k_clap_f32<4, 0, true>, optin),
+      opt_in(k_clap_f32<8, 24, false>, optin), opt_in(k_clap_f32<8, 24, true>, optin),
+      opt_in(k_clap_f32<8, 0, false>, optin),  opt_in(k_clap_f32<8, 0, true>, optin),
+      opt_in(k_batch_clap<24>, optin),         opt_in(k_batch_clap<0>, optin),
+  };
+  for (const cudaError_t x : steps)
+    if (x != cudaSuccess) return x;
+  return cudaSuccess;
+}
+
+}  // namespace ps2

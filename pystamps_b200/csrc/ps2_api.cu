@@ -561,7 +561,7 @@ int enqueue_iteration(ps2_ctx* c, bool later, bool force_continue, cudaEvent_t* 
   CK(launch_bin(bin_args(c, 0, c->K[0].p), fp64, c->sm_count, c->st));
   ++launched;
   if (ev) CK(cudaEventRecord(ev[1], c->st));
-  CK(launch_clap(clap_args_loop(c, c->grid.p, c->clap_fused), fp64, c->twf, c->twd, c->sm_count, c->st));
+  CK(launch_clap(clap_args_loop(c, c->grid.p, c->clap_fused), fp64, c->twd, c->sm_count, c->st));
   OverlapArgs ov = overlap_args_loop(c, c->filt.p, c->clap_fused);
   ov.normalize = fp64 ? 0 : 1;
   CK(launch_overlap(ov, fp64, c->st));
@@ -1171,7 +1171,7 @@ int ps2_autotune(ps2_ctx* c, int32_t* chosen_lanes, double* ms_per_candidate) {
           double ms = 0;
           rc = timed(
               [&] {
-                const cudaError_t e = launch_clap(ca, c->fp64, c->twf, c->twd, c->sm_count, c->st);
+                const cudaError_t e = launch_clap(ca, c->fp64, c->twd, c->sm_count, c->st);
                 return e != cudaSuccess ? e : launch_overlap(ov, c->fp64, c->st);
               },
               &ms);
@@ -1644,7 +1644,7 @@ int ps2_clap_filter_grid(const float* ph_grid, int64_t n_i, int64_t n_j, int64_t
   Twiddles32d td;
   twiddles(&tf, &td);
   if (W > 0) {
-    CK(launch_clap(a, false, tf, td, sc.sm, sc.st));
+    CK(launch_clap(a, false, td, sc.sm, sc.st));
     OverlapArgs o{};
     o.win_out = win.p;
     o.filt = filt.p;
@@ -1846,7 +1846,7 @@ int ps2_clap_filter_grid_noalloc(const float* d_ph_grid, int64_t n_i, int64_t n_
     Twiddles32f tf;
     Twiddles32d td;
     twiddles(&tf, &td);
-    CK(launch_clap(a, false, tf, td, sms, st));
+    CK(launch_clap(a, false, td, sms, st));
     OverlapArgs o{};
     o.win_out = win;
     o.filt = filt;
@@ -1920,7 +1920,7 @@ int coh_prologue(ps2_ctx* c, const float* d_ph, const float* d_K, const float* d
   ca.beta = beta;
   ca.alpha_is_one = alpha == 1.0 ? 1 : 0;
   if (c->nwi > 0 && c->nwj > 0) {
-    CK(launch_clap(ca, fp64, c->twf, c->twd, c->sm_count, st));
+    CK(launch_clap(ca, fp64, c->twd, c->sm_count, st));
     CK(launch_overlap(overlap_args(c, c->ad_win.p, c->ad_filt.p), fp64, st));
   } else {
     CK(cudaMemsetAsync(c->ad_filt.p, 0, Cz * G * c->Mp, st));
@@ -2093,6 +2093,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   plan.ov_prefix.assign(1, 0);
   plan.ps_prefix.assign(1, 0);
   int64_t cap_iter = 1;
+  bool win24 = true;
   for (int64_t p = 0; p < n; ++p) {
     ps2_ctx* c = ctxs[p];
     PatchDev& d = plan.patch[p];
@@ -2118,7 +2119,8 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
     plan.bin_prefix.push_back(plan.bin_prefix.back() + c->G * c->nchunk);
     const int64_t clap_units = c->clap_fused ? static_cast<int64_t>(clap_block_count(c->nwi)) * clap_block_count(c->nwj)
                                              : static_cast<int64_t>(c->nwi) * c->nwj;
-    plan.clap_prefix.push_back(plan.clap_prefix.back() + clap_units * (c->Mp / 4));
+    plan.clap_prefix.push_back(plan.clap_prefix.back() + clap_units * batch_clap_groups(c->Mp));
+    win24 = win24 && c->n_win == 24;
     plan.ov_prefix.push_back(plan.ov_prefix.back() + c->G * c->Mp);
     plan.ps_prefix.push_back(plan.ps_prefix.back() + c->N);
     cap_iter = std::max<int64_t>(cap_iter, std::max<int64_t>(c->max_iter, 1) + 1);
@@ -2167,7 +2169,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   auto enqueue = [&]() -> int {
     CK(launch_batch_begin(b, plan.ps_prefix.back(), c0->sm_count, st));
     CK(launch_batch_bin(b, plan.bin_prefix.back(), c0->sm_count, st));
-    CK(launch_batch_clap(b, plan.clap_prefix.back(), c0->twf, c0->sm_count, st));
+    CK(launch_batch_clap(b, plan.clap_prefix.back(), win24, c0->sm_count, st));
     CK(launch_batch_overlap(b, plan.ov_prefix.back(), c0->sm_count, st));
     for (int cls = 0; cls < 4; ++cls) {
       if (plan.units[cls].empty()) continue;
@@ -2590,7 +2592,7 @@ int ps2_shard_filter(ps2_ctx* c, const void* d_grid, int64_t cell_lo, int64_t ce
         ca.w_lo = ix_lo * c->nwj;
         ca.w_n = (ix_hi - ix_lo + 1) * c->nwj;
       }
-      CK(launch_clap(ca, fp64, c->twf, c->twd, c->sm_count, c->st));
+      CK(launch_clap(ca, fp64, c->twd, c->sm_count, c->st));
     }
   }
   if (cell_hi > cell_lo) {

@@ -315,11 +315,6 @@ template <>
 struct ClapShape<4> {
   static constexpr int kPad = 8;
 };
-template <>
-struct ClapShape<8> {
-  static constexpr int kPad = 4;
-};
-
 __device__ __forceinline__ uint32_t to_bits(float v) { return __float_as_uint(v); }
 __device__ __forceinline__ unsigned long long to_bits(double v) {
   return static_cast<unsigned long long>(__double_as_longlong(v));
@@ -621,33 +616,12 @@ __device__ __forceinline__ void clap_consts(const ClapArgs& a, R* lp, R* wt) {
 template <typename R>
 struct ClapIo;
 template <>
-struct ClapIo<float> {
-  static constexpr int kPer = 2;  // interferograms per access
-  static constexpr int kU = 8;    // accesses in flight per thread
-};
-template <>
 struct ClapIo<double> {
   static constexpr int kPer = 1;
   static constexpr int kU = 4;
 };
 
-// Interferograms c and c + 1 (columns >= M read as zero; only columns < M
-// are dereferenced).
-__device__ __forceinline__ void clap_fetch(const float2* p, const int c, const int M, float (&v)[4]) {
-  if (c + 1 < M) {
-    const float4 q = *reinterpret_cast<const float4*>(p);
-    v[0] = q.x;
-    v[1] = q.y;
-    v[2] = q.z;
-    v[3] = q.w;
-  } else {
-    const float2 q = c < M ? *p : make_float2(0.f, 0.f);
-    v[0] = q.x;
-    v[1] = q.y;
-    v[2] = 0.f;
-    v[3] = 0.f;
-  }
-}
+// Interferogram c (columns >= M read as zero and are not dereferenced).
 __device__ __forceinline__ void clap_fetch(const double2* p, const int c, const int M, double (&v)[2]) {
   const double2 q = c < M ? *p : make_double2(0.0, 0.0);
   v[0] = q.x;
@@ -704,13 +678,7 @@ __device__ __forceinline__ void clap_store_tiles(const ClapArgs& a, const Tile* 
     const int c = NW * g + q0;
     if (c >= a.Mp) continue;
     typename CT<R>::C* dst = out + (wi * nw2 + pix) * a.Mp + c;
-    if constexpr (PER == 2) {
-      // Mp is a multiple of 4 and c even: c + 1 < Mp, 16-byte aligned
-      *reinterpret_cast<float4*>(dst) = make_float4(tiles[q0].re[li][lj], tiles[q0].im[li][lj],
-                                                    tiles[q0 + 1].re[li][lj], tiles[q0 + 1].im[li][lj]);
-    } else {
-      *dst = mk(tiles[q0].re[li][lj], tiles[q0].im[li][lj]);
-    }
+    *dst = mk(tiles[q0].re[li][lj], tiles[q0].im[li][lj]);
   }
 }
 
@@ -798,13 +766,6 @@ __device__ __forceinline__ void clap_task(const ClapArgs& a, const int64_t task,
 // order and rounds once. The window stack of the two-pass form (1.1 GB for a
 // 256 x 256 x 150 grid) is never written; the partials are 2.7x the grid and a
 // block's box stays in L2 while its windows run.
-constexpr int kClapBlockWin = 4;
-__host__ __device__ inline int clap_box(int n_win) {
-  const int n_inc = n_win / 4 > 1 ? n_win / 4 : 1;
-  return (kClapBlockWin - 1) * n_inc + n_win;
-}
-__host__ __device__ inline int clap_block_rows(int nw_axis) { return (nw_axis + kClapBlockWin - 1) / kClapBlockWin; }
-
 // Add (or store, for a cell no earlier window of the block covered) the
 // weighted window in the tiles to the block partial. Box corner (r0, c0); pi1 /
 // pj1 the corner row / column of the block's previous window row / column
@@ -908,12 +869,9 @@ __device__ __forceinline__ ClapSmem<R, NW> clap_smem(unsigned char* raw, const t
   return m;
 }
 
-// FUSED: window blocks into the partials (the loop's form); otherwise windows
-// into the window stack. FP32 blocks are held to the registers that let as
-// many of them reside as their shared memory does (two of eight warps, three
-// of four).
+// FUSED: window blocks into the partials; otherwise windows into the window stack.
 template <typename R, int NW, int NWIN, bool FUSED>
-__global__ void __launch_bounds__(32 * NW, sizeof(R) == 4 ? (NW == 8 ? 2 : 3) : 1)
+__global__ void __launch_bounds__(32 * NW, 1)
     k_clap(ClapArgs a, typename CT<R>::Tw tw) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const ClapSmem<R, NW> m = clap_smem<R, NW>(smem_raw, tw);
@@ -971,13 +929,10 @@ static cudaError_t launch_clap_nw(const ClapArgs& a, const typename CT<R>::Tw& t
   return a.n_win == 24 ? launch_clap_nwin<R, NW, 24>(a, tw, sm_count, st) : launch_clap_nwin<R, NW, 0>(a, tw, sm_count, st);
 }
 
-// FP32: 8 warps per block by default (16 resident warps per SM, shared memory
-// bound), 4 when the launch shape asks for it; FP64: 4 (its tiles are twice the
-// size). Every window's arithmetic is the same whatever the shape.
-cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32f& tf, const Twiddles32d& td, int sm_count,
-                        cudaStream_t st) {
-  if (fp64) return launch_clap_nw<double, 4>(a, td, sm_count, st);
-  return a.nw_block == 4 ? launch_clap_nw<float, 4>(a, tf, sm_count, st) : launch_clap_nw<float, 8>(a, tf, sm_count, st);
+// FP32 is in clap_f32.cu. Every window's
+// arithmetic is the same whatever the shape.
+cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32d& td, int sm_count, cudaStream_t st) {
+  return fp64 ? launch_clap_nw<double, 4>(a, td, sm_count, st) : launch_clap_f32(a, sm_count, st);
 }
 
 // Overlap-add as a gather: cell (i, j) sums the windows that cover it, in the
@@ -3273,18 +3228,6 @@ cudaError_t launch_hist_centers(const double* v, int64_t n, const double* mids, 
 // patch by binary search. Each unit runs the single-patch code on its patch's
 // arguments, so a patch's results do not depend on what it is batched with.
 
-__device__ __forceinline__ int find_patch(const int64_t* __restrict__ prefix, int P, int64_t u) {
-  int lo = 0, hi = P - 1;
-  while (lo < hi) {
-    const int mid = (lo + hi + 1) >> 1;
-    if (prefix[mid] <= u)
-      lo = mid;
-    else
-      hi = mid - 1;
-  }
-  return lo;
-}
-
 // k_iter_begin over the active patches: their statistics cleared (a block per
 // patch), K[1] <- K[0] and the P-square weights from iteration 2 on (elements
 // numbered patch after patch over the whole grid). A block per patch copying its
@@ -3320,30 +3263,6 @@ __global__ void __launch_bounds__(256) k_batch_bin(BatchArgs b) {
     const int p = find_patch(b.bin_prefix, b.P, u);
     if (!b.active[p]) continue;
     bin_task<float>(b.patch[p].bin, u - b.bin_prefix[p], lane);
-  }
-}
-
-__global__ void __launch_bounds__(128) k_batch_clap(BatchArgs b, Twiddles32f tw) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const ClapSmem<float, 4> m = clap_smem<float, 4>(smem_raw, tw);
-  float g7[7];
-  int cur = -1;
-  const int64_t total = b.clap_prefix[b.P];
-  for (int64_t u = blockIdx.x; u < total; u += gridDim.x) {
-    const int p = find_patch(b.clap_prefix, b.P, u);
-    if (!b.active[p]) continue;
-    const ClapArgs& a = b.patch[p].clap;
-    if (p != cur) {
-      // the previous task's readers of lp / wt passed its last barrier
-      clap_consts<float>(a, m.lp, m.wt);
-#pragma unroll
-      for (int i = 0; i < 7; ++i) g7[i] = static_cast<float>(a.g7[i]);
-      cur = p;
-    }
-    if (a.part)
-      clap_block_task<float, 4>(a, u - b.clap_prefix[p], m.tiles, m.twf, m.twi, m.lp, m.wt, g7);
-    else
-      clap_task<float, 4>(a, u - b.clap_prefix[p], m.tiles, m.twf, m.twi, m.lp, m.wt, g7);
   }
 }
 
@@ -3404,20 +3323,6 @@ cudaError_t launch_batch_begin(const BatchArgs& b, int64_t total_ps, int sm_coun
 cudaError_t launch_batch_bin(const BatchArgs& b, int64_t total, int sm_count, cudaStream_t st) {
   const int64_t blocks = std::max<int64_t>(1, std::min<int64_t>((total + 7) / 8, static_cast<int64_t>(sm_count) * 16));
   k_batch_bin<<<static_cast<unsigned>(blocks), 256, 0, st>>>(b);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_batch_clap(const BatchArgs& b, int64_t total, const Twiddles32f& tf, int sm_count,
-                              cudaStream_t st) {
-  if (total <= 0) return cudaSuccess;
-  const size_t sm = clap_smem_bytes<float, 4>();
-  cudaError_t e = kernel_attributes_once(sm);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_clap, 128, sm);
-  if (e != cudaSuccess) return e;
-  const int64_t blocks = std::min<int64_t>(total, static_cast<int64_t>(sm_count) * std::max(per_sm, 1));
-  k_batch_clap<<<static_cast<unsigned>(blocks), 128, sm, st>>>(b, tf);
   return cudaGetLastError();
 }
 
@@ -4176,17 +4081,10 @@ cudaError_t kernel_attributes_once(size_t dynamic_smem) {
     const cudaError_t r = cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
     const cudaError_t steps[] = {
         r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 8, 0, false>, optin) : r,
+        r == cudaSuccess ? clap_f32_attributes(optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 0, false>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 8, 24, false>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 4, 0, false>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 4, 24, false>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 24, false>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 8, 0, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 0, true>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 8, 24, true>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 4, 0, true>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap<float, 4, 24, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 24, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_f32<4>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_f32<8>, optin) : r,
@@ -4198,7 +4096,6 @@ cudaError_t kernel_attributes_once(size_t dynamic_smem) {
         r == cudaSuccess ? opt_in_smem(k_s3_fit, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<float>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<double>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_batch_clap, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_batch_topofit<4>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_batch_topofit<8>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_batch_topofit<16>, optin) : r,

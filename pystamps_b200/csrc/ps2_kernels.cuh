@@ -74,6 +74,15 @@ struct OverlapArgs {
   int64_t cell_lo, cell_n;  // cells cell_lo .. cell_lo + cell_n - 1 (cell_n = 0: all cells)
 };
 
+// The fused form takes the windows in blocks of 4 x 4, whose cells lie in a box of
+// clap_box(n_win) a side (clap_accum_tiles).
+constexpr int kClapBlockWin = 4;
+__host__ __device__ inline int clap_box(int n_win) {
+  const int n_inc = n_win / 4 > 1 ? n_win / 4 : 1;
+  return (kClapBlockWin - 1) * n_inc + n_win;
+}
+__host__ __device__ inline int clap_block_rows(int nw_axis) { return (nw_axis + kClapBlockWin - 1) / kClapBlockWin; }
+
 // --------------------------------------------------------------- topofit --
 struct TopoArgs {
   const void* ph_nm;      // complex [N, M] sorted (loop mode)
@@ -180,10 +189,23 @@ struct BatchArgs {
   int* active;                // [P] 1 while the patch iterates
   int* n_active;              // [1]
   const int64_t* bin_prefix;  // [P + 1] warp-tasks (G * nchunk)
-  const int64_t* clap_prefix; // [P + 1] block-tasks (W * Mp / 4)
+  const int64_t* clap_prefix; // [P + 1] block-tasks (windows or window blocks x interferogram groups)
   const int64_t* ov_prefix;   // [P + 1] elements (G * Mp)
   const int64_t* ps_prefix;   // [P + 1] PS
 };
+
+// the patch of unit u (prefix: [P + 1])
+__device__ __forceinline__ int find_patch(const int64_t* __restrict__ prefix, int P, int64_t u) {
+  int lo = 0, hi = P - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (prefix[mid] <= u)
+      lo = mid;
+    else
+      hi = mid - 1;
+  }
+  return lo;
+}
 
 // -------------------------------------------------------------- adjoints --
 // R-typed arrays are float or double by the context's precision.
@@ -215,8 +237,11 @@ struct ClapBwdArgs {
 // ---------------------------------------------------------- launchers -----
 cudaError_t launch_bin(const BinArgs& a, bool fp64, int sm_count, cudaStream_t st);
 cudaError_t launch_iter_begin(const BeginArgs& a, bool fp64, int sm_count, cudaStream_t st);
-cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32f& tf, const Twiddles32d& td, int sm_count,
-                        cudaStream_t st);
+cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32d& td, int sm_count, cudaStream_t st);
+cudaError_t launch_clap_f32(const ClapArgs& a, int sm_count, cudaStream_t st);
+cudaError_t clap_f32_attributes(int optin);
+// block-tasks per window of a batch's CLAP (8 interferograms each)
+int64_t batch_clap_groups(int Mp);
 cudaError_t launch_overlap(const OverlapArgs& a, bool fp64, cudaStream_t st);
 cudaError_t launch_topofit(const TopoArgs& a, bool fp64, int grid_blocks, cudaStream_t st);
 int topofit_grid_blocks(int sm_count, bool fp64);
@@ -267,8 +292,7 @@ cudaError_t launch_topofit_near_max(const NearMaxArgs& a, bool fp64, int sm_coun
 cudaError_t launch_hist_centers(const double* v, int64_t n, const double* mids, int nc, int equal, double d,
                                 double cutoff0, unsigned long long* counts, int sm_count, cudaStream_t st);
 cudaError_t launch_batch_bin(const BatchArgs& b, int64_t total, int sm_count, cudaStream_t st);
-cudaError_t launch_batch_clap(const BatchArgs& b, int64_t total, const Twiddles32f& tf, int sm_count,
-                              cudaStream_t st);
+cudaError_t launch_batch_clap(const BatchArgs& b, int64_t total, bool win24, int sm_count, cudaStream_t st);
 cudaError_t launch_batch_overlap(const BatchArgs& b, int64_t total, int sm_count, cudaStream_t st);
 cudaError_t launch_batch_topofit(const BatchArgs& b, int L, const int32_t* units, int n_units, size_t smem,
                                  int sm_count, cudaStream_t st);

@@ -12,8 +12,8 @@ pytestmark = pytest.mark.gpu
 
 # columns around the 8 lanes and the 32-lane rounds, up to the largest; trials
 # around the blocks of 8 magnitudes; rows around the 4 of a warp and the 8 of a block
-CASES = [(1, 41, 9, False), (7, 1, 300, False), (7, 3, 301, True), (8, 17, 302, False), (9, 19, 303, True), (31, 41, 200, False),
-         (33, 81, 201, True), (64, 33, 202, False), (150, 175, 100, False), (256, 35, 61, False)]
+CASES = [(1, 41, 297, False), (7, 1, 300, False), (7, 3, 301, True), (8, 17, 302, False), (9, 19, 303, True), (31, 41, 200, False),
+         (33, 81, 201, True), (64, 33, 202, False), (150, 175, 100, False), (256, 35, 121, False)]
 
 
 @pytest.mark.parametrize("m,trials,n,same_baseline", CASES)
@@ -21,7 +21,7 @@ def test_trial_and_refinement(cuda_lib, m, trials, n, same_baseline):
     from pystamps_b200 import stage2 as S
     from pystamps_b200 import synth
 
-    patch = synth.make_patch(n, max(m, 3), 24, 41, seed=100 + m, n_rand=1000)
+    patch = synth.make_patch(n, max(m, 3), 28, 41, seed=100 + m, n_rand=1000)
     p = S.prepare_patch(patch, nr=np.ones(100))
     half = (trials - 1) // 2
     bp = np.ascontiguousarray(p.bperp[:, :m])
