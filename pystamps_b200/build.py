@@ -4,12 +4,14 @@ from __future__ import annotations
 import os
 import shutil
 import subprocess
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
 HERE = Path(__file__).resolve().parent
 CSRC = HERE / "csrc"
-SOURCES = [CSRC / "ps2_kernels.cu", CSRC / "ps2_api.cu", CSRC / "clap_f32.cu", CSRC / "v5_uniform.cu"]
-HEADERS = [CSRC / "ps2_kernels.cuh", CSRC / "ps2_device.cuh", CSRC / "v5_uniform.cuh", CSRC / "clap_f32.cuh", CSRC / "interp10_taps.h", CSRC / "trial_interp_taps.h", CSRC / "sincos_poly.h", CSRC / "atan_poly.h",
+SOURCES = [CSRC / "ps2_kernels.cu", CSRC / "ps2_api.cu", CSRC / "clap_f32.cu", CSRC / "topofit_f32.cu", CSRC / "v5_uniform.cu"]
+HEADERS = [CSRC / "ps2_kernels.cuh", CSRC / "ps2_device.cuh", CSRC / "v5_uniform.cuh", CSRC / "clap_f32.cuh", CSRC / "phase_math.cuh", CSRC / "interp10_taps.h", CSRC / "trial_interp_taps.h", CSRC / "sincos_poly.h", CSRC / "atan_poly.h",
            HERE.parent / "include" / "ps2cuda.h"]
 TARGET = HERE / "libps2cuda.so"
 
@@ -36,10 +38,13 @@ def needs_build() -> bool:
 def build(force: bool = False, verbose: bool = False) -> Path:
     if not force and not needs_build():
         return TARGET
-    cmd = [nvcc(), *NVCC_FLAGS, "-o", str(TARGET), *map(str, SOURCES)]
-    if verbose:
-        cmd.insert(1, "-Xptxas=-v")
-    subprocess.run(cmd, check=True, cwd=str(HERE))
+    flags = [f for f in NVCC_FLAGS if f != "-shared"] + (["-Xptxas=-v"] if verbose else [])
+    with tempfile.TemporaryDirectory() as tmp:  # one object per source, compiled side by side
+        objs = [str(Path(tmp) / (s.stem + ".o")) for s in SOURCES]
+        with ThreadPoolExecutor(len(SOURCES)) as ex:
+            list(ex.map(lambda so: subprocess.run([nvcc(), *flags, "-c", "-o", so[1], str(so[0])], check=True, cwd=str(HERE)),
+                        zip(SOURCES, objs)))
+        subprocess.run([nvcc(), *NVCC_FLAGS, "-o", str(TARGET), *objs], check=True, cwd=str(HERE))
     return TARGET
 
 

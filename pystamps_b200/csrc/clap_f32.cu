@@ -332,15 +332,6 @@ cudaError_t launch_nw(const ClapArgs& a, int sm_count, cudaStream_t st) {
                 : launch_form<NW, 0, false>(a, ntask, sm_count, st);
 }
 
-template <typename F>
-cudaError_t opt_in(F* f, int optin) {
-  cudaFuncAttributes fa;
-  cudaError_t e = cudaFuncGetAttributes(&fa, f);
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              optin - static_cast<int>(fa.sharedSizeBytes));
-}
-
 }  // namespace
 
 int64_t batch_clap_groups(int Mp) { return groups_f<8>(Mp); }
@@ -364,11 +355,11 @@ cudaError_t launch_batch_clap(const BatchArgs& b, int64_t total, bool win24, int
 
 cudaError_t clap_f32_attributes(int optin) {
   const cudaError_t steps[] = {
-      opt_in(k_clap_f32<4, 24, false>, optin), opt_in(k_clap_f32<4, 24, true>, optin),
-      opt_in(k_clap_f32<4, 0, false>, optin),  opt_in(k_clap_f32<4, 0, true>, optin),
-      opt_in(k_clap_f32<8, 24, false>, optin), opt_in(k_clap_f32<8, 24, true>, optin),
-      opt_in(k_clap_f32<8, 0, false>, optin),  opt_in(k_clap_f32<8, 0, true>, optin),
-      opt_in(k_batch_clap<24>, optin),         opt_in(k_batch_clap<0>, optin),
+      opt_in_smem(k_clap_f32<4, 24, false>, optin), opt_in_smem(k_clap_f32<4, 24, true>, optin),
+      opt_in_smem(k_clap_f32<4, 0, false>, optin),  opt_in_smem(k_clap_f32<4, 0, true>, optin),
+      opt_in_smem(k_clap_f32<8, 24, false>, optin), opt_in_smem(k_clap_f32<8, 24, true>, optin),
+      opt_in_smem(k_clap_f32<8, 0, false>, optin),  opt_in_smem(k_clap_f32<8, 0, true>, optin),
+      opt_in_smem(k_batch_clap<24>, optin),         opt_in_smem(k_batch_clap<0>, optin),
   };
   for (const cudaError_t x : steps)
     if (x != cudaSuccess) return x;

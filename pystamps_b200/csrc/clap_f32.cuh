@@ -13,12 +13,12 @@
 // rounded cosine, 6e-17, is below the rounding of any sum it would enter).
 #pragma once
 
+#include "phase_math.cuh"
 #include "ps2_device.cuh"
 #include "ps2_kernels.cuh"
 
 namespace ps2 {
 
-__device__ __forceinline__ float2 both(const float v) { return make_float2(v, v); }
 __device__ __forceinline__ float2 sub2(const float2 a, const float2 b) {
   float2 r;
   asm("{.reg .b64 a, b, c; mov.b64 a, {%2, %3}; mov.b64 b, {%4, %5}; sub.rn.f32x2 c, a, b; mov.b64 {%0, %1}, c;}"
@@ -38,23 +38,6 @@ static __constant__ float kSin32[16] = {
     0x1.6a09e60000000p-1f, 0x1.a9b6620000000p-1f, 0x1.d906bc0000000p-1f, 0x1.f6297c0000000p-1f,
     0x1.0000000000000p+0f, 0x1.f6297c0000000p-1f, 0x1.d906bc0000000p-1f, 0x1.a9b6620000000p-1f,
     0x1.6a09e60000000p-1f, 0x1.1c73b40000000p-1f, 0x1.87de2a0000000p-2f, 0x1.8f8b840000000p-3f};
-
-// Square roots of two values by one Newton step from the reciprocal square root
-// approximation: y ~ 1 / sqrt(q), s = q y, s + (q - s^2) y / 2 with the residual exact
-// in one FMA. Equal to sqrtf for every float in [2^-100, infinity) (all 1.9e9 bit
-// patterns compared); outside, callers take sqrtf itself. 5 instructions a value
-// against 25 for sqrtf, whose range checks branch value by value: magnitudes were
-// a fifth of a window's time.
-constexpr uint32_t kSqrtLo = 0x0d800000u;                // 2^-100
-constexpr uint32_t kSqrtSpan = 0x7f800000u - kSqrtLo;  // up to infinity
-__device__ __forceinline__ float2 sqrt_newton2(const float2 q) {
-  float2 y;
-  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y.x) : "f"(q.x));
-  asm("rsqrt.approx.f32 %0, %1;" : "=f"(y.y) : "f"(q.y));
-  const float2 s = __fmul2_rn(q, y), h = __fmul2_rn(both(0.5f), y);
-  const float2 r = __ffma2_rn(make_float2(-s.x, -s.y), s, q);
-  return __ffma2_rn(r, h, s);
-}
 
 // One window of one interferogram. Rows of 34 floats: a lane reads its own row in
 // 8-byte accesses and writes a column, both without bank conflicts; the pad

@@ -2093,7 +2093,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
   plan.ov_prefix.assign(1, 0);
   plan.ps_prefix.assign(1, 0);
   int64_t cap_iter = 1;
-  bool win24 = true;
+  bool win24 = true, rowvar = true;
   for (int64_t p = 0; p < n; ++p) {
     ps2_ctx* c = ctxs[p];
     PatchDev& d = plan.patch[p];
@@ -2121,6 +2121,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
                                              : static_cast<int64_t>(c->nwi) * c->nwj;
     plan.clap_prefix.push_back(plan.clap_prefix.back() + clap_units * batch_clap_groups(c->Mp));
     win24 = win24 && c->n_win == 24;
+    rowvar = rowvar && !c->bp_row_inv;
     plan.ov_prefix.push_back(plan.ov_prefix.back() + c->G * c->Mp);
     plan.ps_prefix.push_back(plan.ps_prefix.back() + c->N);
     cap_iter = std::max<int64_t>(cap_iter, std::max<int64_t>(c->max_iter, 1) + 1);
@@ -2174,7 +2175,7 @@ int ps2_batch_run(ps2_ctx* const* ctxs, int64_t n, ps2_iter_stats* last) {
     for (int cls = 0; cls < 4; ++cls) {
       if (plan.units[cls].empty()) continue;
       CK(launch_batch_topofit(b, lanes_of[cls], reinterpret_cast<const int32_t*>(base + o_cls[cls]),
-                              static_cast<int>(plan.units[cls].size() / 2), plan.smem_max[cls], c0->sm_count, st));
+                              static_cast<int>(plan.units[cls].size() / 2), plan.smem_max[cls], rowvar, c0->sm_count, st));
     }
     CK(launch_batch_finalize(b, st));
     return PS2_OK;

@@ -68,6 +68,19 @@ __device__ __forceinline__ double warp_max(double v) {
   return v;
 }
 
+// sum over the L lanes of a group
+template <int L>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
+}
+template <int L>
+__device__ __forceinline__ double group_sum(double v) {
+#pragma unroll
+  for (int o = L / 2; o > 0; o >>= 1) v += __shfl_xor_sync(kFull, v, o);
+  return v;
+}
 // Histogram bin of the equal-spacing Octave rule used for the coherence
 // histogram (native_stage2.rs:1593-1607): centres 0.005 + 0.01*i, i < 100.
 // d and cutoff0 are computed on the host exactly like the reference.

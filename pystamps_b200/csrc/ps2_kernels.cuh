@@ -234,12 +234,24 @@ struct ClapBwdArgs {
   double* ab_partial;   // [2 * blocks]: d L / d alpha, d L / d beta per block
 };
 
+// a kernel may take the device's whole shared memory per block, less its static part
+template <typename F>
+inline cudaError_t opt_in_smem(F* f, int optin) {
+  cudaFuncAttributes fa;
+  cudaError_t e = cudaFuncGetAttributes(&fa, f);
+  if (e != cudaSuccess) return e;
+  return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              optin - static_cast<int>(fa.sharedSizeBytes));
+}
+
 // ---------------------------------------------------------- launchers -----
 cudaError_t launch_bin(const BinArgs& a, bool fp64, int sm_count, cudaStream_t st);
 cudaError_t launch_iter_begin(const BeginArgs& a, bool fp64, int sm_count, cudaStream_t st);
 cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32d& td, int sm_count, cudaStream_t st);
 cudaError_t launch_clap_f32(const ClapArgs& a, int sm_count, cudaStream_t st);
 cudaError_t clap_f32_attributes(int optin);
+cudaError_t launch_topofit_f32(const TopoArgs& a, int grid_blocks, cudaStream_t st);
+cudaError_t topofit_f32_attributes(int optin);
 // block-tasks per window of a batch's CLAP (8 interferograms each)
 int64_t batch_clap_groups(int Mp);
 cudaError_t launch_overlap(const OverlapArgs& a, bool fp64, cudaStream_t st);
@@ -294,7 +306,7 @@ cudaError_t launch_hist_centers(const double* v, int64_t n, const double* mids, 
 cudaError_t launch_batch_bin(const BatchArgs& b, int64_t total, int sm_count, cudaStream_t st);
 cudaError_t launch_batch_clap(const BatchArgs& b, int64_t total, bool win24, int sm_count, cudaStream_t st);
 cudaError_t launch_batch_overlap(const BatchArgs& b, int64_t total, int sm_count, cudaStream_t st);
-cudaError_t launch_batch_topofit(const BatchArgs& b, int L, const int32_t* units, int n_units, size_t smem,
+cudaError_t launch_batch_topofit(const BatchArgs& b, int L, const int32_t* units, int n_units, size_t smem, bool rowvar,
                                  int sm_count, cudaStream_t st);
 cudaError_t launch_batch_finalize(const BatchArgs& b, cudaStream_t st);
 cudaError_t launch_batch_continue(cudaGraphConditionalHandle h, const int* n_active, cudaStream_t st);
