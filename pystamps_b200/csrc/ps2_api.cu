@@ -2385,7 +2385,8 @@ int ps3_reestimate(const ps3_reestimate_desc* d, ps3_reestimate_out* o, int devi
   ca.low_pass = lp.as<double>();
   gauss7(ca.g7, nullptr);
   ca.job_out = jout.as<float2>();
-  CK(launch_s3_clap(ca, tf, sc.sm, st));
+  ca.quarter_cos = tf.w[8].x;
+  CK(launch_s3_clap(ca, sc.sm, st));
   S3FitArgs fa{};
   fa.ph = ph.as<float2>();
   fa.bp = bp.as<float>();
@@ -2499,7 +2500,8 @@ int ps2_stage3_reestimate(ps2_ctx* c, const int64_t* sel, int64_t n_sel, const i
   ca.low_pass = c->low_pass.as<double>();
   gauss7(ca.g7, nullptr);
   ca.job_out = jout.as<float2>();
-  CK(launch_s3_clap(ca, c->twf, c->sm_count, st));
+  ca.quarter_cos = c->twf.w[8].x;
+  CK(launch_s3_clap(ca, c->sm_count, st));
   S3FitArgs fa{};
   fa.ph = c->ph_nm.as<float2>();
   fa.bp = c->bp.as<float>();

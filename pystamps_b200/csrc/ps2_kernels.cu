@@ -1704,133 +1704,6 @@ cudaError_t launch_random_hist(const double* rnd, int64_t n_rand, const double* 
 // the filtered value at that cell is kept; then each selected PS is re-fitted
 // (_ps_topofit_single, :2355-2431) against it.
 
-// One warp: the 32x32 patch in its tile -> the filtered value at (bi, bj),
-// times 1024. The inverse FFT is evaluated at that one point:
-// y = sum_{k1,k2} Y[k1][k2] e^{+2 pi i (k1 bi + k2 bj) / 32}.
-__device__ __forceinline__ float2 s3_patch_point(ClapTile<float>& T, const int lane, const S3ClapArgs& a,
-                                                 const float2* twf, const float2* wp, const float* lp,
-                                                 const float (&g7)[7], const int bi, const int bj) {
-  fft_pass<float>(T.re, T.im, twf, lane, true);
-  __syncwarp();
-  fft_pass<float>(T.re, T.im, twf, lane, false);
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const float xr = T.re[k][lane], xi = T.im[k][lane];
-    T.hs[k][lane] = sqrtf(xr * xr + xi * xi);
-  }
-  __syncwarp();
-  // 7x7 Gaussian 'same' smoothing of fftshift(|X|), then ifftshift, in
-  // unshifted coordinates (the seam at the Nyquist row / column)
-  float t[32];
-  const int sj = (lane + 16) & 31;
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    float acc = 0.f;
-#pragma unroll
-    for (int d = -3; d <= 3; ++d)
-      if (sj + d >= 0 && sj + d < 32) acc += T.hs[k][(lane + d) & 31] * g7[d + 3];
-    t[k] = acc;
-  }
-  float o[32];
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const int sk = (k + 16) & 31;
-    float acc = 0.f;
-#pragma unroll
-    for (int d = -3; d <= 3; ++d)
-      if (sk + d >= 0 && sk + d < 32) acc += t[(k + d) & 31] * g7[d + 3];
-    o[k] = acc;
-  }
-  const float med = warp_median1024<float>(o, &T.hs[0][0]);
-  const float beta = static_cast<float>(a.beta), alpha = static_cast<float>(a.alpha);
-  const float inv_med = med != 0.f ? 1.f / med : 1.f;
-  float2 acc = make_float2(0.f, 0.f);
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    float v = o[k] * inv_med;
-    v = a.alpha_is_one ? v - 1.f : powf(v, alpha) - 1.f;
-    if (v < 0.f) v = 0.f;
-    const float gk = v * beta + lp[k * 32 + lane];
-    const float2 y = make_float2(T.re[k][lane] * gk, T.im[k][lane] * gk);
-    const float2 w = wp[(k * bi) & 31];
-    acc.x += y.x * w.x - y.y * w.y;
-    acc.y += y.x * w.y + y.y * w.x;
-  }
-  const float2 w = wp[(lane * bj) & 31];
-  float2 r = make_float2(acc.x * w.x - acc.y * w.y, acc.x * w.y + acc.y * w.x);
-  r.x = warp_sum(r.x);
-  r.y = warp_sum(r.y);
-  return r;
-}
-
-__global__ void __launch_bounds__(128) k_s3_clap(S3ClapArgs a, Twiddles32f tw) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  ClapTile<float>* tiles = reinterpret_cast<ClapTile<float>*>(smem_raw);
-  float* lp = reinterpret_cast<float*>(tiles + 4);
-  float2* twf = reinterpret_cast<float2*>(lp + 1024);
-  float2* wp = twf + 16;  // e^{+2 pi i k / 32}, k < 32
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  for (int i = tid; i < 1024; i += 128) lp[i] = static_cast<float>(a.low_pass[i]);
-  if (tid < 16) {
-    twf[tid] = tw.w[tid];
-    wp[tid] = make_float2(tw.w[tid].x, -tw.w[tid].y);
-    wp[tid + 16] = make_float2(-tw.w[tid].x, tw.w[tid].y);
-  }
-  float g7[7];
-#pragma unroll
-  for (int i = 0; i < 7; ++i) g7[i] = static_cast<float>(a.g7[i]);
-  const int M = a.M;
-  const int64_t ntask = a.n_jobs * a.ngroups;
-  for (int64_t task = blockIdx.x; task < ntask; task += gridDim.x) {
-    const int64_t job = task / a.ngroups;
-    const int g = static_cast<int>(task - job * a.ngroups);
-    const int i0 = a.jobs[4 * job], j0 = a.jobs[4 * job + 1], bi = a.jobs[4 * job + 2], bj = a.jobs[4 * job + 3];
-    const int c_warp = 4 * g + warp;
-    if (i0 < 0) {
-      // the 32-cell patch does not fit: the reference sets ph_patch2 to 0
-      if (lane == 0 && c_warp < M) a.job_out[job * M + c_warp] = make_float2(0.f, 0.f);
-      continue;
-    }
-    __syncthreads();
-    for (int idx = tid; idx < 4 * 1024; idx += 128) {
-      const int pix = idx >> 2, q = idx & 3;
-      const int li = pix >> 5, lj = pix & 31;
-      const int c = 4 * g + q;
-      float2 v = make_float2(0.f, 0.f);
-      if (c < M) {
-        v = a.grid[(static_cast<int64_t>(i0 + li) * a.grid_cols + (j0 + lj)) * a.grid_stride + c];
-        if (isnan(v.x) || isnan(v.y)) v = make_float2(0.f, 0.f);
-        const bool own = li == bi && lj == bj;
-        const bool osf = c == 0 && abs(li - bi) <= a.slc_rad && abs(lj - bj) <= a.slc_rad;
-        if (own || osf) v = make_float2(0.f, 0.f);
-      }
-      tiles[q].re[li][lj] = v.x;
-      tiles[q].im[li][lj] = v.y;
-    }
-    __syncthreads();
-    if (c_warp < M) {
-      const float2 r = s3_patch_point(tiles[warp], lane, a, twf, wp, lp, g7, bi, bj);
-      if (lane == 0) a.job_out[job * M + c_warp] = make_float2(r.x * (1.f / 1024.f), r.y * (1.f / 1024.f));
-    }
-  }
-}
-
-size_t s3_clap_smem() { return 4 * sizeof(ClapTile<float>) + 1024 * sizeof(float) + 48 * sizeof(float2); }
-
-cudaError_t launch_s3_clap(const S3ClapArgs& a, const Twiddles32f& tf, int sm_count, cudaStream_t st) {
-  const int64_t ntask = a.n_jobs * a.ngroups;
-  if (ntask <= 0) return cudaSuccess;
-  const size_t sm = s3_clap_smem();
-  cudaError_t e = kernel_attributes_once(sm);
-  if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_s3_clap, 128, sm);
-  if (e != cudaSuccess) return e;
-  const int64_t blocks = std::min<int64_t>(ntask, static_cast<int64_t>(sm_count) * std::max(per_sm, 1));
-  k_s3_clap<<<static_cast<unsigned>(blocks), 128, sm, st>>>(a, tf);
-  return cudaGetLastError();
-}
-
 // np.exp(-1j * x) in complex64: (cos x, -sin x)
 __device__ __forceinline__ float2 s3_cis_neg(float x) {
   float s, c;
@@ -3103,7 +2976,6 @@ cudaError_t kernel_attributes_once(size_t dynamic_smem) {
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 24, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_f64, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_random_hist, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_s3_clap, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_s3_fit, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<float>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<double>, optin) : r,

@@ -149,6 +149,7 @@ struct S3ClapArgs {
   const double* low_pass;  // [32 * 32]
   double g7[7];
   float2* job_out;         // [n_jobs, M] filtered value at the PS cell
+  float quarter_cos;       // cos(pi / 2) as the twiddle tables round it (6e-17)
 };
 
 struct S3FitArgs {
@@ -280,7 +281,7 @@ int64_t clap_part_elems(int nwi, int nwj, int n_win, int Mp);
 int clap_block_count(int nw_axis);
 cudaError_t topofit_geometry(const TopoArgs& a, int grid_cap, int* L_out, int* mpad_out, int* blocks_out);
 cudaError_t launch_batch_begin(const BatchArgs& b, int64_t total_ps, int sm_count, cudaStream_t st);
-cudaError_t launch_s3_clap(const S3ClapArgs& a, const Twiddles32f& tf, int sm_count, cudaStream_t st);
+cudaError_t launch_s3_clap(const S3ClapArgs& a, int sm_count, cudaStream_t st);
 cudaError_t launch_s3_fit(const S3FitArgs& a, int sm_count, cudaStream_t st);
 
 // ----------------------------------------------------- registry topofit --
