@@ -481,7 +481,7 @@ TopoArgs topo_args(ps2_ctx* c, void* K_out, void* C_out, void* coh_io) {
   t.Mp = c->Mp;
   t.n_half = c->n_half;
   t.zero_mode = 0;
-  t.filt_unit = c->fp64 ? 0 : 1;  // the loop's k_overlap stores f/|f| in FP32
+  t.filt_unit = 1;  // the loop's k_overlap stores f/|f|
   t.K_out = K_out;
   t.C_out = C_out;
   t.coh_io = coh_io;
@@ -563,7 +563,7 @@ int enqueue_iteration(ps2_ctx* c, bool later, bool force_continue, cudaEvent_t* 
   if (ev) CK(cudaEventRecord(ev[1], c->st));
   CK(launch_clap(clap_args_loop(c, c->grid.p, c->clap_fused), fp64, c->twd, c->sm_count, c->st));
   OverlapArgs ov = overlap_args_loop(c, c->filt.p, c->clap_fused);
-  ov.normalize = fp64 ? 0 : 1;
+  ov.normalize = 1;
   CK(launch_overlap(ov, fp64, c->st));
   launched += 2;
   if (ev) CK(cudaEventRecord(ev[2], c->st));
@@ -1167,7 +1167,7 @@ int ps2_autotune(ps2_ctx* c, int32_t* chosen_lanes, double* ms_per_candidate) {
           ca.nw_block = c->fp64 ? 0 : nws[a];
           ca.blocks_per_sm = bpss[b];
           OverlapArgs ov = overlap_args_loop(c, c->filt.p, f);
-          ov.normalize = c->fp64 ? 0 : 1;
+          ov.normalize = 1;
           double ms = 0;
           rc = timed(
               [&] {
@@ -2600,7 +2600,7 @@ int ps2_shard_filter(ps2_ctx* c, const void* d_grid, int64_t cell_lo, int64_t ce
   }
   if (cell_hi > cell_lo) {
     OverlapArgs ov = overlap_args_loop(c, c->filt.p, c->clap_fused);
-    ov.normalize = fp64 ? 0 : 1;
+    ov.normalize = 1;
     ov.cell_lo = cell_lo;
     ov.cell_n = cell_hi - cell_lo;
     CK(launch_overlap(ov, fp64, c->st));

@@ -936,13 +936,11 @@ __device__ __forceinline__ void overlap_elem(const OverlapArgs& a, const int64_t
       }
     }
     C f = mk(static_cast<R>(sx), static_cast<R>(sy));
-    if constexpr (sizeof(R) == 4) {
-      if (a.normalize) {
-        // normalize_complex_unit_magnitude (:1186-1205) once per cell instead of
-        // once per PS of the cell in the topofit; the same expression, the same bits
-        const float mag = hypotf(f.x, f.y);
-        if (mag != 0.f) f = make_float2(f.x / mag, f.y / mag);
-      }
+    if (a.normalize) {
+      // normalize_complex_unit_magnitude (:1186-1205) once per cell instead of
+      // once per PS of the cell in the topofit; the same expression, the same bits
+      const R mag = hypot_r(f.x, f.y);
+      if (mag != R(0)) f = mk(f.x / mag, f.y / mag);
     }
     filt[idx] = f;
   }
@@ -985,11 +983,9 @@ __device__ __forceinline__ void combine_elem(const OverlapArgs& a, const int64_t
     }
   }
   C f = mk(static_cast<R>(sx), static_cast<R>(sy));
-  if constexpr (sizeof(R) == 4) {
-    if (a.normalize) {
-      const float mag = hypotf(f.x, f.y);
-      if (mag != 0.f) f = make_float2(f.x / mag, f.y / mag);
-    }
+  if (a.normalize) {
+    const R mag = hypot_r(f.x, f.y);
+    if (mag != R(0)) f = mk(f.x / mag, f.y / mag);
   }
   filt[idx] = f;
 }
@@ -1029,7 +1025,7 @@ cudaError_t launch_overlap(const OverlapArgs& a, bool fp64, cudaStream_t st) {
 // chains only rank the trials: where the best one does not lead by more than
 // their rounding error, the row's trials are evaluated again by the direct sum
 // (every lane its trials, columns in order), so the trial chosen is the direct
-// sum's. 100,000 PS x 40 ifg x 121 trials: 1.73 -> 0.69 ms.
+// sum's. 100,000 PS x 40 ifg x 121 trials: 1.73 -> 0.57 ms.
 constexpr int kF64Lanes = 8, kF64Ps = 32 / kF64Lanes, kF64Warps = 2, kF64W = 8;
 
 // Row stride in columns: M padded to the lanes, an odd multiple of 8 so that the
@@ -1069,6 +1065,7 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
   __shared__ int sh_hist[kCohBins];
   __shared__ double sh_rms[kF64Warps];
   __shared__ int sh_inv[kF64Warps];
+  __shared__ double sh_row[kF64Warps][kF64Ps][4];  // per row: range, trial K, refined K, sums
   for (int i = tid; i < kCohBins; i += blockDim.x) sh_hist[i] = 0;
   __syncthreads();
   const float2* __restrict__ ph_nm = static_cast<const float2*>(a.ph_nm);
@@ -1090,25 +1087,31 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
   for (int64_t s0 = gw * kF64Ps; s0 < a.N; s0 += nwarps * kF64Ps) {
     const int rows = a.N - s0 < kF64Ps ? static_cast<int>(a.N - s0) : kF64Ps;
     unsigned invalid_rows = 0;
-    double range_g = 1.0;  // of the lane's own row in the sweep
+    __syncwarp();
+    // elementwise steps run over all elements of the rows, so that no lane idles at
+    // the end of each row
+    const int total = rows * a.M;
+    for (int idx = lane; idx < total; idx += 32) {
+      const int q = idx / a.M, c = idx - q * a.M;
+      const int64_t s = s0 + q, cell = a.cell_of[s];
+      double2 f = filt[cell * a.Mp + c];
+      if (!a.filt_unit) {
+        const double mag = hypot(f.x, f.y);
+        if (mag != 0.0) f = make_double2(f.x / mag, f.y / mag);
+      }
+      if (ph_patch) ph_patch[s * M + c] = f;
+      const float2 p = ph_nm[s * M + c];
+      zs0[q * stride + c] = cmul_rn(conjd2(f), make_double2(p.x, p.y));
+      rot0[q * stride + c].x = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
+    }
     __syncwarp();
     for (int q = 0; q < rows; ++q) {
-      const int64_t s = s0 + q, cell = a.cell_of[s];
-      double2* zs = zs0 + q * stride;
-      double2* rot = rot0 + q * stride;
       bool zero = false;
       double mn = INFINITY, mx = -INFINITY;
       for (int c = lane; c < a.M; c += 32) {
-        double2 f = filt[cell * a.Mp + c];
-        const double mag = hypot(f.x, f.y);
-        if (mag != 0.0) f = make_double2(f.x / mag, f.y / mag);
-        if (ph_patch) ph_patch[s * M + c] = f;
-        const float2 p = ph_nm[s * M + c];
-        const double2 v = cmul_rn(conjd2(f), make_double2(p.x, p.y));
-        zs[c] = v;
+        const double2 v = zs0[q * stride + c];
         if (v.x == 0.0 && v.y == 0.0) zero = true;
-        const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
-        rot[c].x = b;
+        const double b = rot0[q * stride + c].x;
         mn = fmin(mn, b);
         mx = fmax(mx, b);
       }
@@ -1117,17 +1120,18 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
       mx = warp_max(mx);
       double range = mx - mn;
       if (range == 0.0) range = 1.0;
-      if (g == q) range_g = range;
-      __syncwarp();
-      for (int c = lane; c < mpad; c += 32) {
-        const bool in = c < a.M;
-        const double th = in ? (rot[c].x / range) * qpi : 0.0;
-        if (!in) zs[c] = make_double2(0.0, 0.0);
-        double sn, cs;
-        sincos(th, &sn, &cs);
-        rot[c] = make_double2(cs, -sn);
-        ph0[q * stride + c] = make_double2(cs, -sn);  // |m| = 1
-      }
+      if (lane == 0) sh_row[wib][q][0] = range;
+    }
+    __syncwarp();
+    for (int idx = lane; idx < rows * mpad; idx += 32) {
+      const int q = idx / mpad, c = idx - q * mpad;
+      const bool in = c < a.M;
+      const double th = in ? (rot0[q * stride + c].x / sh_row[wib][q][0]) * qpi : 0.0;
+      if (!in) zs0[q * stride + c] = make_double2(0.0, 0.0);
+      double sn, cs;
+      sincos(th, &sn, &cs);
+      rot0[q * stride + c] = make_double2(cs, -sn);
+      ph0[q * stride + c] = make_double2(cs, -sn);  // |m| = 1
     }
     __syncwarp();
     // trial chains of row s0 + g over the lane's columns gl, gl + 8, ...: with
@@ -1219,117 +1223,150 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
       const int64_t s = s0 + q;
       const double2* zs = zs0 + q * stride;
       double2* rot = rot0 + q * stride;
-      const double range = __shfl_sync(kFull, range_g, q * kF64Lanes);
+      const double range = sh_row[wib][q][0];
       int bt = __shfl_sync(kFull, top.t, q * kF64Lanes);
-      double Kv, Cv, cohv;
-      if ((invalid_rows >> q) & 1u) {
-        Kv = __longlong_as_double(0x7ff8000000000000LL);
-        Cv = 0.0;
-        cohv = 0.0;
+      if (!((invalid_rows >> q) & 1u) && !((clear >> (q * kF64Lanes)) & 1u)) {
         for (int c = lane; c < a.M; c += 32) {
-          if (resid) resid[s * M + c] = make_double2(0.0, 0.0);
-          if (ph_res) ph_res[s * M + c] = 0.0;
+          const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
+          rot[c].x = (b / range) * qpi;
         }
+        __syncwarp();
+        double best = -1.0;
+        bt = 0;
+        for (int t = lane; t < T; t += 32) {
+          const double m = static_cast<double>(t - a.n_half);
+          double sx = 0.0, sy = 0.0;
+          for (int c = 0; c < a.M; ++c) {
+            double sn, cs;
+            sincos(rot[c].x * m, &sn, &cs);
+            const double2 z = zs[c];
+            sx += z.x * cs + z.y * sn;
+            sy += z.y * cs - z.x * sn;
+          }
+          const double sq = sx * sx + sy * sy;
+          if (sq > best) {
+            best = sq;
+            bt = t;
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const double ob = __shfl_xor_sync(kFull, best, o);
+          const int ot = __shfl_xor_sync(kFull, bt, o);
+          if (ob > best || (ob == best && ot < bt)) {
+            best = ob;
+            bt = ot;
+          }
+        }
+        __syncwarp();
+      }
+      if (lane == 0) sh_row[wib][q][1] = qpi / range * static_cast<double>(bt - a.n_half);
+    }
+    __syncwarp();
+    auto bperp = [&](int64_t s, int c) {
+      return a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
+    };
+    // refine_candidate (native_stage2.rs:1259-1303): elements of all rows, then each
+    // row's sums (lanes over its columns)
+    for (int idx = lane; idx < total; idx += 32) {
+      const int q = idx / a.M, c = idx - q * a.M;
+      double sn, cs;
+      sincos(sh_row[wib][q][1] * bperp(s0 + q, c), &sn, &cs);
+      rot0[q * stride + c] = cmul_rn(zs0[q * stride + c], make_double2(cs, -sn));
+    }
+    __syncwarp();
+    for (int q = 0; q < rows; ++q) {
+      double ox = 0.0, oy = 0.0;
+      for (int c = lane; c < a.M; c += 32) {
+        ox += rot0[q * stride + c].x;
+        oy += rot0[q * stride + c].y;
+      }
+      ox = warp_sum(ox);
+      oy = warp_sum(oy);
+      if (lane == 0) {
+        sh_row[wib][q][2] = ox;
+        sh_row[wib][q][3] = oy;
+      }
+    }
+    __syncwarp();
+    for (int idx = lane; idx < total; idx += 32) {
+      const int q = idx / a.M, c = idx - q * a.M;
+      const double2 z = zs0[q * stride + c];
+      const double wgt = hypot(z.x, z.y);
+      const double2 x = cmul_rn(rot0[q * stride + c], make_double2(sh_row[wib][q][2], -sh_row[wib][q][3]));
+      ph0[q * stride + c] = make_double2(wgt * bperp(s0 + q, c), wgt * atan2(x.y, x.x));
+    }
+    __syncwarp();
+    for (int q = 0; q < rows; ++q) {
+      double mopt = 0.0, dl = 0.0;
+      for (int c = lane; c < a.M; c += 32) {
+        const double2 x = ph0[q * stride + c];
+        dl = fma(x.x, x.x, dl);
+        mopt = fma(x.x, x.y, mopt);
+      }
+      mopt = warp_sum(mopt);
+      dl = warp_sum(dl);
+      if (dl == 0.0) dl = 1.0;
+      if (lane == 0) sh_row[wib][q][2] = sh_row[wib][q][1] + mopt / dl;
+    }
+    __syncwarp();
+    for (int idx = lane; idx < total; idx += 32) {
+      const int q = idx / a.M, c = idx - q * a.M;
+      const int64_t s = s0 + q;
+      double sn, cs;
+      sincos(sh_row[wib][q][2] * bperp(s, c), &sn, &cs);
+      const double2 r = cmul_rn(zs0[q * stride + c], make_double2(cs, -sn));
+      rot0[q * stride + c] = r;
+      ph0[q * stride + c].x = hypot(r.x, r.y);
+      const bool bad = (invalid_rows >> q) & 1u;
+      if (resid) resid[s * M + c] = bad ? make_double2(0.0, 0.0) : r;
+      if (ph_res) ph_res[s * M + c] = bad ? 0.0 : atan2(r.y, r.x);
+    }
+    __syncwarp();
+    double mx2 = 0.0, my2 = 0.0, den2 = 0.0;  // of row s0 + lane
+    for (int q = 0; q < rows; ++q) {
+      double x = 0.0, y = 0.0, d = 0.0;
+      for (int c = lane; c < a.M; c += 32) {
+        x += rot0[q * stride + c].x;
+        y += rot0[q * stride + c].y;
+        d += ph0[q * stride + c].x;
+      }
+      x = warp_sum(x);
+      y = warp_sum(y);
+      d = warp_sum(d);
+      if (lane == q) {
+        mx2 = x;
+        my2 = y;
+        den2 = d;
+      }
+    }
+    if (lane < rows) {
+      const int64_t s = s0 + lane;
+      const bool bad = (invalid_rows >> lane) & 1u;
+      double Kv = __longlong_as_double(0x7ff8000000000000LL), Cv = 0.0, cohv = 0.0;
+      if (bad) {
         inv_acc += 1;
       } else {
-        if (!((clear >> (q * kF64Lanes)) & 1u)) {
-          for (int c = lane; c < a.M; c += 32) {
-            const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
-            rot[c].x = (b / range) * qpi;
-          }
-          __syncwarp();
-          double best = -1.0;
-          bt = 0;
-          for (int t = lane; t < T; t += 32) {
-            const double m = static_cast<double>(t - a.n_half);
-            double sx = 0.0, sy = 0.0;
-            for (int c = 0; c < a.M; ++c) {
-              double sn, cs;
-              sincos(rot[c].x * m, &sn, &cs);
-              const double2 z = zs[c];
-              sx += z.x * cs + z.y * sn;
-              sy += z.y * cs - z.x * sn;
-            }
-            const double sq = sx * sx + sy * sy;
-            if (sq > best) {
-              best = sq;
-              bt = t;
-            }
-          }
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) {
-            const double ob = __shfl_xor_sync(kFull, best, o);
-            const int ot = __shfl_xor_sync(kFull, bt, o);
-            if (ob > best || (ob == best && ot < bt)) {
-              best = ob;
-              bt = ot;
-            }
-          }
-          __syncwarp();
-        }
-        const double k0 = qpi / range * static_cast<double>(bt - a.n_half);
-        double ox = 0.0, oy = 0.0;
-        for (int c = lane; c < a.M; c += 32) {
-          const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
-          double sn, cs;
-          sincos(k0 * b, &sn, &cs);
-          const double2 r = cmul_rn(zs[c], make_double2(cs, -sn));
-          rot[c] = r;
-          ox += r.x;
-          oy += r.y;
-        }
-        ox = warp_sum(ox);
-        oy = warp_sum(oy);
-        double mopt = 0.0, dl = 0.0;
-        for (int c = lane; c < a.M; c += 32) {
-          const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
-          const double2 r = rot[c];
-          const double wgt = hypot(zs[c].x, zs[c].y);
-          const double wb = wgt * b;
-          dl += wb * wb;
-          const double2 q = cmul_rn(r, make_double2(ox, -oy));
-          mopt += wb * (wgt * atan2(q.y, q.x));
-        }
-        mopt = warp_sum(mopt);
-        dl = warp_sum(dl);
-        if (dl == 0.0) dl = 1.0;
-        const double K1 = k0 + mopt / dl;
-        double mx2 = 0.0, my2 = 0.0, den2 = 0.0;
-        for (int c = lane; c < a.M; c += 32) {
-          const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
-          double sn, cs;
-          sincos(K1 * b, &sn, &cs);
-          const double2 r = cmul_rn(zs[c], make_double2(cs, -sn));
-          mx2 += r.x;
-          my2 += r.y;
-          den2 += hypot(r.x, r.y);
-          if (resid) resid[s * M + c] = r;
-          if (ph_res) ph_res[s * M + c] = atan2(r.y, r.x);
-        }
-        mx2 = warp_sum(mx2);
-        my2 = warp_sum(my2);
-        den2 = warp_sum(den2);
         if (den2 == 0.0) den2 = 1.0;
-        Kv = K1;
+        Kv = sh_row[wib][lane][2];
         Cv = atan2(my2, mx2);
         cohv = hypot(mx2, my2) / den2;
       }
-      __syncwarp();
-      if (lane == 0) {
-        if (a.accumulate_stats) {
-          const double d = cohv - coh_io[s];
-          rms_acc += d * d;
-          const int b = coh_bin(cohv, a.cutoff0, a.dbin);
-          if (b >= 0) atomicAdd(&sh_hist[b], 1);
-        }
-        K_out[s] = Kv;
-        C_out[s] = Cv;
-        coh_io[s] = cohv;
-        if (a.nopt) a.nopt[s] = ((invalid_rows >> q) & 1u) ? 0 : 1;
+      if (a.accumulate_stats) {
+        const double d = cohv - coh_io[s];
+        rms_acc += d * d;
+        const int b = coh_bin(cohv, a.cutoff0, a.dbin);
+        if (b >= 0) atomicAdd(&sh_hist[b], 1);
       }
+      K_out[s] = Kv;
+      C_out[s] = Cv;
+      coh_io[s] = cohv;
+      if (a.nopt) a.nopt[s] = bad ? 0 : 1;
     }
   }
   if (!a.accumulate_stats) return;
+  rms_acc = warp_sum(rms_acc);
+  inv_acc = warp_sum(inv_acc);
   if (lane == 0) {
     sh_rms[wib] = rms_acc;
     sh_inv[wib] = inv_acc;
@@ -1562,17 +1599,27 @@ __global__ void __launch_bounds__(256) k_trial_phasors(const double* __restrict_
   }
 }
 
-__global__ void __launch_bounds__(256) k_random_hist(const double* __restrict__ rnd, int64_t n_rand,
-                                                     const double* __restrict__ bp, int m,
-                                                     const int64_t* __restrict__ ia, const int64_t* __restrict__ ib,
-                                                     int small_baseline, int n_half, double cutoff0, double dbin,
-                                                     const double2* __restrict__ E, int32_t* hist) {
+// A warp takes R rows: their trial sums run together (lanes over trials, each
+// phasor of the table read once for R rows, columns in order), the trials ranked by
+// |S|^2; a row whose two largest lie within rounding is decided by |S| / m as the
+// reference compares it. The refinement's elementwise steps run over all elements
+// of the R rows, its ordered sums side by side, one lane a chain (by themselves
+// three chains of m dependent additions a row, the whole warp waiting). Bound by
+// the FP64 pipe: 6 operations per (row, trial, column). 300,000 rows x 60 x 161
+// trials: 4.4 -> 2.55 ms.
+constexpr int kHistWarps = 4;
+template <int R>
+__global__ void __launch_bounds__(32 * kHistWarps) k_random_hist(
+    const double* __restrict__ rnd, int64_t n_rand, const double* __restrict__ bp, int m,
+    const int64_t* __restrict__ ia, const int64_t* __restrict__ ib, int small_baseline, int n_half, double cutoff0,
+    double dbin, const double2* __restrict__ E, int32_t* hist) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-  double* ph = reinterpret_cast<double*>(smem_raw) + static_cast<int64_t>(wib) * 3 * m;
-  double* t1 = ph + m;
-  double* t2 = t1 + m;
+  double2* u = reinterpret_cast<double2*>(smem_raw) + static_cast<int64_t>(wib) * R * m;
+  double* ph = reinterpret_cast<double*>(reinterpret_cast<double2*>(smem_raw) + static_cast<int64_t>(kHistWarps) * R * m) +
+               static_cast<int64_t>(wib) * R * m;
   __shared__ int sh_hist[kCohBins];
+  __shared__ double sh_k[kHistWarps][R], sh_sum[kHistWarps][R][2];
   for (int i = tid; i < kCohBins; i += blockDim.x) sh_hist[i] = 0;
   __syncthreads();
   const int T = 2 * n_half + 1;
@@ -1586,90 +1633,148 @@ __global__ void __launch_bounds__(256) k_random_hist(const double* __restrict__ 
   const double qpi = 3.14159265358979323846 / 4.0;
   const int64_t gw = (static_cast<int64_t>(blockIdx.x) * blockDim.x + tid) >> 5;
   const int64_t nw = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  for (int64_t row = gw; row < n_rand; row += nw) {
+  // the sum of one component of row r over the columns, in order, by lane 2 r + s
+  auto ordered_sums = [&]() {
     __syncwarp();
-    for (int c = lane; c < m; c += 32)
-      ph[c] = small_baseline ? rnd[row + ib[c] * n_rand] - rnd[row + ia[c] * n_rand] : rnd[row + c * n_rand];
-    // e^{j ph_c} once per row; the trial sum of e^{j (ph_c - theta_c m)} is then
-    // e^{j ph_c} e^{-j theta_c m} from the phasor table: 4 FP64 operations per
-    // (trial, column) instead of a sincos (the terms differ from sincos of the
-    // rounded angle in the last bit; the sums keep the column order)
-    for (int c = lane; c < m; c += 32) {
-      double sn, cs;
-      sincos(ph[c], &sn, &cs);
-      t1[c] = cs;
-      t2[c] = sn;
+    if (lane < 2 * R) {
+      const double2* x = u + (lane >> 1) * m;
+      double acc = 0.0;
+      if (lane & 1)
+        for (int c = 0; c < m; ++c) acc = __dadd_rn(acc, x[c].y);
+      else
+        for (int c = 0; c < m; ++c) acc = __dadd_rn(acc, x[c].x);
+      sh_sum[wib][lane >> 1][lane & 1] = acc;
     }
     __syncwarp();
-    double best = -1.0;
-    int bt = 0;
-    for (int t = lane; t < T; t += 32) {
-      double sre = 0.0, sim = 0.0;
-      for (int c = 0; c < m; ++c) {
-        const double2 e = E[static_cast<int64_t>(c) * T + t];
-        const double cp = t1[c], sp = t2[c];
-        sre = __dadd_rn(sre, __fma_rn(cp, e.x, __dmul_rn(sp, e.y)));
-        sim = __dadd_rn(sim, __fma_rn(sp, e.x, -__dmul_rn(cp, e.y)));
-      }
-      const double v = hypot(sre, sim) / static_cast<double>(m);
-      if (v > best) {
-        best = v;
-        bt = t;
+  };
+  for (int64_t row0 = gw * R; row0 < n_rand; row0 += nw * R) {
+    __syncwarp();
+    // e^{j ph_c} of the rows (rows past the end repeat the last one)
+    for (int idx = lane; idx < R * m; idx += 32) {
+      const int c = idx / R, r = idx % R;
+      const int64_t row = row0 + r < n_rand ? row0 + r : n_rand - 1;
+      const double p = small_baseline ? rnd[row + ib[c] * n_rand] - rnd[row + ia[c] * n_rand] : rnd[row + c * n_rand];
+      double sn, cs;
+      sincos(p, &sn, &cs);
+      ph[r * m + c] = p;
+      u[r * m + c] = make_double2(cs, sn);
+    }
+    __syncwarp();
+    Top2 top[R];
+#pragma unroll
+    for (int r = 0; r < R; ++r) top[r] = Top2{-1.0, -1.0, 0};
+    for (int t0 = 0; t0 < T; t0 += 32) {
+      const int rem = T - t0;
+      if (rem * R <= 32) {
+        // the last few trials: a lane for each (row, trial)
+        constexpr int PER = 32 / R;
+        const int rr = lane / PER, j = lane % PER, t = t0 + (j < rem ? j : 0);
+        double sre = 0.0, sim = 0.0;
+        for (int c = 0; c < m; ++c) {
+          const double2 e = E[static_cast<int64_t>(c) * T + t], w = u[rr * m + c];
+          sre = __dadd_rn(sre, __fma_rn(w.x, e.x, __dmul_rn(w.y, e.y)));
+          sim = __dadd_rn(sim, __fma_rn(w.y, e.x, -__dmul_rn(w.x, e.y)));
+        }
+        const double sq = __fma_rn(sre, sre, __dmul_rn(sim, sim));
+#pragma unroll
+        for (int r = 0; r < R; ++r)
+          if (r == rr && j < rem) top[r].add(sq, t);
+      } else {
+        const int t = t0 + lane < T ? t0 + lane : T - 1;
+        double sre[R], sim[R];
+#pragma unroll
+        for (int r = 0; r < R; ++r) sre[r] = sim[r] = 0.0;
+#pragma unroll 4
+        for (int c = 0; c < m; ++c) {
+          const double2 e = E[static_cast<int64_t>(c) * T + t];
+#pragma unroll
+          for (int r = 0; r < R; ++r) {
+            const double2 w = u[r * m + c];
+            sre[r] = __dadd_rn(sre[r], __fma_rn(w.x, e.x, __dmul_rn(w.y, e.y)));
+            sim[r] = __dadd_rn(sim[r], __fma_rn(w.y, e.x, -__dmul_rn(w.x, e.y)));
+          }
+        }
+        if (t0 + lane < T) {
+#pragma unroll
+          for (int r = 0; r < R; ++r) top[r].add(__fma_rn(sre[r], sre[r], __dmul_rn(sim[r], sim[r])), t);
+        }
       }
     }
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double ob = __shfl_xor_sync(kFull, best, o);
-      const int ot = __shfl_xor_sync(kFull, bt, o);
-      if (ob > best || (ob == best && ot < bt)) {
-        best = ob;
-        bt = ot;
+    for (int r = 0; r < R; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(kFull, top[r].best, o), os = __shfl_xor_sync(kFull, top[r].second, o);
+        const int ot = __shfl_xor_sync(kFull, top[r].t, o);
+        const bool theirs = ob > top[r].best || (ob == top[r].best && ot < top[r].t);
+        top[r].second = fmax(theirs ? top[r].best : ob, theirs ? os : top[r].second);
+        if (theirs) {
+          top[r].best = ob;
+          top[r].t = ot;
+        }
       }
+      int bt = top[r].t;
+      if (!(top[r].best - top[r].second > 1.0e-13 * top[r].best)) {
+        // |S| / m as compared by the reference (topofit_phase_row_coh)
+        double best = -1.0;
+        bt = 0;
+        for (int t = lane; t < T; t += 32) {
+          double sre = 0.0, sim = 0.0;
+          for (int c = 0; c < m; ++c) {
+            const double2 e = E[static_cast<int64_t>(c) * T + t], w = u[r * m + c];
+            sre = __dadd_rn(sre, __fma_rn(w.x, e.x, __dmul_rn(w.y, e.y)));
+            sim = __dadd_rn(sim, __fma_rn(w.y, e.x, -__dmul_rn(w.x, e.y)));
+          }
+          const double v = hypot(sre, sim) / static_cast<double>(m);
+          if (v > best) {
+            best = v;
+            bt = t;
+          }
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          const double ob = __shfl_xor_sync(kFull, best, o);
+          const int ot = __shfl_xor_sync(kFull, bt, o);
+          if (ob > best || (ob == best && ot < bt)) {
+            best = ob;
+            bt = ot;
+          }
+        }
+      }
+      if (lane == 0) sh_k[wib][r] = qpi / range * static_cast<double>(bt - n_half);
     }
-    const double k0 = qpi / range * static_cast<double>(bt - n_half);
-    for (int c = lane; c < m; c += 32) {
+    __syncwarp();
+    for (int idx = lane; idx < R * m; idx += 32) {
+      const int r = idx / m, c = idx - r * m;
       double sn, cs;
-      sincos(__dsub_rn(ph[c], __dmul_rn(k0, bp[c])), &sn, &cs);
-      t1[c] = cs;
-      t2[c] = sn;
+      sincos(__dsub_rn(ph[idx], __dmul_rn(sh_k[wib][r], bp[c])), &sn, &cs);
+      u[idx] = make_double2(cs, sn);
     }
-    __syncwarp();
-    double ore = 0.0, oim = 0.0;
-    for (int c = 0; c < m; ++c) {
-      ore = __dadd_rn(ore, t1[c]);
-      oim = __dadd_rn(oim, t2[c]);
-    }
-    __syncwarp();
-    for (int c = lane; c < m; c += 32) {
-      const double cs = t1[c], sn = t2[c];
+    ordered_sums();
+    for (int idx = lane; idx < R * m; idx += 32) {
+      const int r = idx / m, c = idx - r * m;
+      const double cs = u[idx].x, sn = u[idx].y, ore = sh_sum[wib][r][0], oim = sh_sum[wib][r][1];
       const double pre = __dsub_rn(__dmul_rn(cs, ore), __dmul_rn(sn, -oim));
       const double pim = __dadd_rn(__dmul_rn(cs, -oim), __dmul_rn(sn, ore));
-      t1[c] = __dmul_rn(bp[c], atan2(pim, pre));
-      t2[c] = __dmul_rn(bp[c], bp[c]);
+      u[idx] = make_double2(__dmul_rn(bp[c], atan2(pim, pre)), __dmul_rn(bp[c], bp[c]));
+    }
+    ordered_sums();
+    if (lane < R) {
+      const double mopt = sh_sum[wib][lane][0];
+      double den = sh_sum[wib][lane][1];
+      if (den == 0.0) den = 1.0;
+      sh_k[wib][lane] = sh_k[wib][lane] + mopt / den;
     }
     __syncwarp();
-    double mopt = 0.0, den = 0.0;
-    for (int c = 0; c < m; ++c) {
-      den = __dadd_rn(den, t2[c]);
-      mopt = __dadd_rn(mopt, t1[c]);
-    }
-    if (den == 0.0) den = 1.0;
-    const double k = k0 + mopt / den;
-    __syncwarp();
-    for (int c = lane; c < m; c += 32) {
+    for (int idx = lane; idx < R * m; idx += 32) {
+      const int r = idx / m, c = idx - r * m;
       double sn, cs;
-      sincos(__dsub_rn(ph[c], __dmul_rn(k, bp[c])), &sn, &cs);
-      t1[c] = cs;
-      t2[c] = sn;
+      sincos(__dsub_rn(ph[idx], __dmul_rn(sh_k[wib][r], bp[c])), &sn, &cs);
+      u[idx] = make_double2(cs, sn);
     }
-    __syncwarp();
-    if (lane == 0) {
-      double sre = 0.0, sim = 0.0;
-      for (int c = 0; c < m; ++c) {
-        sre = __dadd_rn(sre, t1[c]);
-        sim = __dadd_rn(sim, t2[c]);
-      }
-      const double coh = hypot(sre, sim) / static_cast<double>(m > 1 ? m : 1);
+    ordered_sums();
+    if (lane < R && row0 + lane < n_rand) {
+      const double coh = hypot(sh_sum[wib][lane][0], sh_sum[wib][lane][1]) / static_cast<double>(m > 1 ? m : 1);
       const int b = coh_bin(coh, cutoff0, dbin);
       if (b >= 0) atomicAdd(&sh_hist[b], 1);
     }
@@ -1679,21 +1784,32 @@ __global__ void __launch_bounds__(256) k_random_hist(const double* __restrict__ 
     if (sh_hist[i]) atomicAdd(&hist[i], sh_hist[i]);
 }
 
+template <int R>
+static cudaError_t random_hist_rows(const double* rnd, int64_t n_rand, const double* bp, int m, const int64_t* ia,
+                                    const int64_t* ib, int small_baseline, int n_half, double cutoff0, double dbin,
+                                    const double2* phasors, int32_t* hist, int sm_count, cudaStream_t st) {
+  const size_t sm = static_cast<size_t>(kHistWarps) * R * m * (sizeof(double2) + sizeof(double));
+  cudaError_t e = kernel_attributes_once(sm);
+  if (e != cudaSuccess) return e;
+  const int64_t per_block = static_cast<int64_t>(kHistWarps) * R;
+  const int64_t blocks =
+      std::max<int64_t>(1, std::min<int64_t>((n_rand + per_block - 1) / per_block, static_cast<int64_t>(sm_count) * 8));
+  k_random_hist<R><<<static_cast<unsigned>(blocks), 32 * kHistWarps, sm, st>>>(
+      rnd, n_rand, bp, m, ia, ib, small_baseline, n_half, cutoff0, dbin, phasors, hist);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_random_hist(const double* rnd, int64_t n_rand, const double* bp, int m, const int64_t* ia,
                                const int64_t* ib, int small_baseline, int n_half, double cutoff0, double dbin,
                                double2* phasors, int32_t* hist, int sm_count, cudaStream_t st) {
-  const size_t sm = static_cast<size_t>(8) * 3 * m * sizeof(double);
-  cudaError_t e = kernel_attributes_once(sm);
-  if (e != cudaSuccess) return e;
   const int64_t n_ph = static_cast<int64_t>(m) * (2 * n_half + 1);
   k_trial_phasors<<<static_cast<unsigned>(std::min<int64_t>((n_ph + 255) / 256, static_cast<int64_t>(sm_count) * 8)),
                     256, 0, st>>>(bp, m, n_half, phasors);
-  int64_t blocks = (n_rand + 7) / 8;
-  if (blocks > static_cast<int64_t>(sm_count) * 8) blocks = static_cast<int64_t>(sm_count) * 8;
-  if (blocks < 1) blocks = 1;
-  k_random_hist<<<static_cast<unsigned>(blocks), 256, sm, st>>>(rnd, n_rand, bp, m, ia, ib, small_baseline, n_half,
-                                                                cutoff0, dbin, phasors, hist);
-  return cudaGetLastError();
+  // 8 rows a warp up to 64 columns (four blocks an SM), 4 beyond
+  return m <= 64 ? random_hist_rows<8>(rnd, n_rand, bp, m, ia, ib, small_baseline, n_half, cutoff0, dbin, phasors, hist,
+                                       sm_count, st)
+                 : random_hist_rows<4>(rnd, n_rand, bp, m, ia, ib, small_baseline, n_half, cutoff0, dbin, phasors, hist,
+                                       sm_count, st);
 }
 
 
@@ -2842,10 +2958,28 @@ __global__ void k_gather_rows(const uint32_t* __restrict__ src, uint32_t* __rest
   }
 }
 
+// one word a row (per-PS vectors): a thread per element, not a warp
+__global__ void k_gather_words(const uint32_t* __restrict__ src, uint32_t* __restrict__ dst,
+                               const int32_t* __restrict__ perm, int64_t n, int scatter) {
+  for (int64_t s = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; s < n;
+       s += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int64_t r = perm[s];
+    if (scatter)
+      dst[r] = src[s];
+    else
+      dst[s] = src[r];
+  }
+}
+
 static cudaError_t gather_impl(const void* src, void* dst, const int32_t* perm, int64_t n, int64_t row_bytes,
                                int scatter, cudaStream_t st) {
   if (n <= 0) return cudaSuccess;
   if (row_bytes % 4) return cudaErrorInvalidValue;
+  if (row_bytes == 4) {
+    k_gather_words<<<static_cast<unsigned>(std::min<int64_t>((n + 255) / 256, 148 * 8)), 256, 0, st>>>(
+        static_cast<const uint32_t*>(src), static_cast<uint32_t*>(dst), perm, n, scatter);
+    return cudaGetLastError();
+  }
   int64_t blocks = (n + 7) / 8;
   if (blocks > 148 * 16) blocks = 148 * 16;
   k_gather_rows<<<static_cast<unsigned>(blocks), 256, 0, st>>>(static_cast<const uint32_t*>(src),
@@ -2975,7 +3109,8 @@ cudaError_t kernel_attributes_once(size_t dynamic_smem) {
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 0, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 24, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_f64, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_random_hist, optin) : r,
+        r == cudaSuccess ? opt_in_smem(k_random_hist<4>, optin) : r,
+        r == cudaSuccess ? opt_in_smem(k_random_hist<8>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_s3_fit, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<float>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<double>, optin) : r,

@@ -70,7 +70,7 @@ struct OverlapArgs {
   const void* part;     // complex FP64 block partials of the fused form (win_out unused)
   void* filt;           // complex [G, Mp]
   int n_i, n_j, M, Mp, n_win, n_inc, nwi, nwj;
-  int normalize;        // 1 (FP32 stage-2 loop): store f/|f|, the unit patch phase the topofit reads
+  int normalize;        // 1 (stage-2 loop): store f/|f|, the unit patch phase the topofit reads
   int64_t cell_lo, cell_n;  // cells cell_lo .. cell_lo + cell_n - 1 (cell_n = 0: all cells)
 };
 
@@ -109,7 +109,7 @@ struct TopoArgs {
   void* ph_patch;         // complex [N, M]
   int accumulate_stats;   // 1: rms partials / histogram / invalid count
   int lanes;              // lanes per PS in the FP32 kernel (4, 8, 16, 32); 0: from n_ifg
-  int filt_unit;          // 1: filt already holds f/|f| (k_overlap with normalize), FP32 kernel
+  int filt_unit;          // 1: filt already holds f/|f| (k_overlap with normalize)
 };
 
 // -------------------------------------------------------------- finalize --
