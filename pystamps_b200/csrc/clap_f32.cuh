@@ -57,39 +57,63 @@ enum FftPass : int {
   kForward1 = 0,  // own row of the zero-padded window; result transposed
   kForward2 = 1,  // own column of the spectrum; result and (transposed) magnitude
   kInverse1 = 2,  // gain from hs, re and im exchanged; result transposed
-  kInverse2 = 3,  // own row; result left to the caller's epilogue
+  kInverse2 = 3,  // own row; the result times the pyramid weights
+  // the gradient's (FORM 2): without magnitude, gain and weights
+  kForward2Plain = 4,
+  kInverse1Plain = 5,
+  kInverse2Plain = 6,
 };
 
 // The 32-point transform of lane's row of T; pass p of the window (uniform).
 // Window rows and columns >= NZ are zero and, in pass 0, not read. In pass
 // kInverse2 the lane's result times its pyramid weights wt[l] (l < nw) goes back to
 // its row.
-template <int NZ, typename Tile>
+// FORM 0: all four passes; 1: the forward ones (adjoint's window); 2: the plain ones.
+template <int NZ, int FORM = 0, typename Tile>
 __device__ __noinline__ void fft_row(Tile& T, const int lane, const int p, const float* wt, const int rs, const int cs,
                                      const int nw) {
   float2 ar[16], ai[16];  // points 2 m and 2 m + 1 at the bit reversal of m
+  auto at = [](int m) { return ((m & 1) << 3) | ((m & 2) << 1) | ((m & 4) >> 1) | ((m & 8) >> 3); };
+  bool done = false;
   if (p == kForward1) {
+    done = true;
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
-      const int j = ((m & 1) << 3) | ((m & 2) << 1) | ((m & 4) >> 1) | ((m & 8) >> 3);
+      const int j = at(m);
       ar[j] = ai[j] = make_float2(0.f, 0.f);
       if (2 * m < NZ && lane < NZ) {
         ar[j] = *reinterpret_cast<const float2*>(&T.re[lane][2 * m]);
         ai[j] = *reinterpret_cast<const float2*>(&T.im[lane][2 * m]);
       }
     }
-  } else if (p == kInverse1) {
+  }
+  if constexpr (FORM == 0) {
+    if (p == kInverse1) {
+      done = true;
 #pragma unroll
-    for (int m = 0; m < 16; ++m) {
-      const int j = ((m & 1) << 3) | ((m & 2) << 1) | ((m & 4) >> 1) | ((m & 8) >> 3);
-      const float2 g = *reinterpret_cast<const float2*>(&T.hs[lane][2 * m]);
-      ar[j] = __fmul2_rn(*reinterpret_cast<const float2*>(&T.im[lane][2 * m]), g);
-      ai[j] = __fmul2_rn(*reinterpret_cast<const float2*>(&T.re[lane][2 * m]), g);
+      for (int m = 0; m < 16; ++m) {
+        const int j = at(m);
+        const float2 g = *reinterpret_cast<const float2*>(&T.hs[lane][2 * m]);
+        ar[j] = __fmul2_rn(*reinterpret_cast<const float2*>(&T.im[lane][2 * m]), g);
+        ai[j] = __fmul2_rn(*reinterpret_cast<const float2*>(&T.re[lane][2 * m]), g);
+      }
     }
-  } else {
+  }
+  if constexpr (FORM == 2) {
+    if (p == kInverse1Plain) {
+      done = true;
+#pragma unroll
+      for (int m = 0; m < 16; ++m) {
+        const int j = at(m);
+        ar[j] = *reinterpret_cast<const float2*>(&T.im[lane][2 * m]);
+        ai[j] = *reinterpret_cast<const float2*>(&T.re[lane][2 * m]);
+      }
+    }
+  }
+  if (!done) {
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
-      const int j = ((m & 1) << 3) | ((m & 2) << 1) | ((m & 4) >> 1) | ((m & 8) >> 3);
+      const int j = at(m);
       ar[j] = *reinterpret_cast<const float2*>(&T.re[lane][2 * m]);
       ai[j] = *reinterpret_cast<const float2*>(&T.im[lane][2 * m]);
     }
@@ -141,36 +165,55 @@ __device__ __noinline__ void fft_row(Tile& T, const int lane, const int p, const
     xr[k + 16] = __fsub_rn(ur, tr);
     xi[k + 16] = __fsub_rn(ui, tj);
   }
-  if (p == kForward2) {
-    uint32_t far = 0;
+  done = false;
+  if constexpr (FORM != 2) {
+    if (p == kForward2) {
+      done = true;
+      uint32_t far = 0;
 #pragma unroll
-    for (int k = 0; k < 32; k += 2) {
-      const float2 r = make_float2(xr[k], xr[k + 1]), i = make_float2(xi[k], xi[k + 1]);
-      *reinterpret_cast<float2*>(&T.re[lane][k]) = r;
-      *reinterpret_cast<float2*>(&T.im[lane][k]) = i;
-      const float2 q = __ffma2_rn(r, r, __fmul2_rn(i, i));
-      const float2 m = sqrt_newton2(q);
-      T.hs[k][lane] = m.x;
-      T.hs[k + 1][lane] = m.y;
-      far = max(far, max(__float_as_uint(q.x) - kSqrtLo, __float_as_uint(q.y) - kSqrtLo));
-    }
-    if (far >= kSqrtSpan) {  // a zero, a tiny or an infinite value among them
+      for (int k = 0; k < 32; k += 2) {
+        const float2 r = make_float2(xr[k], xr[k + 1]), i = make_float2(xi[k], xi[k + 1]);
+        *reinterpret_cast<float2*>(&T.re[lane][k]) = r;
+        *reinterpret_cast<float2*>(&T.im[lane][k]) = i;
+        const float2 q = __ffma2_rn(r, r, __fmul2_rn(i, i));
+        const float2 m = sqrt_newton2(q);
+        T.hs[k][lane] = m.x;
+        T.hs[k + 1][lane] = m.y;
+        far = max(far, max(__float_as_uint(q.x) - kSqrtLo, __float_as_uint(q.y) - kSqrtLo));
+      }
+      if (far >= kSqrtSpan) {  // a zero, a tiny or an infinite value among them
 #pragma unroll 1
-      for (int k = 0; k < 32; ++k)
-        T.hs[k][lane] = sqrtf(__fmaf_rn(T.re[lane][k], T.re[lane][k], __fmul_rn(T.im[lane][k], T.im[lane][k])));
-    }
-  } else if (p == kInverse2) {
-    if (lane < nw) {
-      const bool row_zero = lane < rs;
-#pragma unroll
-      for (int l = 0; l < NZ; l += 2) {
-        const float2 wv = make_float2((row_zero || l < cs || l >= nw) ? 0.f : wt[l],
-                                      (row_zero || l + 1 < cs || l + 1 >= nw) ? 0.f : wt[l + 1]);
-        *reinterpret_cast<float2*>(&T.re[lane][l]) = __fmul2_rn(make_float2(xr[l], xr[l + 1]), wv);
-        *reinterpret_cast<float2*>(&T.im[lane][l]) = __fmul2_rn(make_float2(xi[l], xi[l + 1]), wv);
+        for (int k = 0; k < 32; ++k)
+          T.hs[k][lane] = sqrtf(__fmaf_rn(T.re[lane][k], T.re[lane][k], __fmul_rn(T.im[lane][k], T.im[lane][k])));
       }
     }
-  } else {
+  }
+  if constexpr (FORM == 0) {
+    if (p == kInverse2) {
+      done = true;
+      if (lane < nw) {
+        const bool row_zero = lane < rs;
+#pragma unroll
+        for (int l = 0; l < NZ; l += 2) {
+          const float2 wv = make_float2((row_zero || l < cs || l >= nw) ? 0.f : wt[l],
+                                        (row_zero || l + 1 < cs || l + 1 >= nw) ? 0.f : wt[l + 1]);
+          *reinterpret_cast<float2*>(&T.re[lane][l]) = __fmul2_rn(make_float2(xr[l], xr[l + 1]), wv);
+          *reinterpret_cast<float2*>(&T.im[lane][l]) = __fmul2_rn(make_float2(xi[l], xi[l + 1]), wv);
+        }
+      }
+    }
+  }
+  if constexpr (FORM == 2) {
+    if (p == kForward2Plain || p == kInverse2Plain) {
+      done = true;
+#pragma unroll
+      for (int k = 0; k < 32; k += 2) {
+        *reinterpret_cast<float2*>(&T.re[lane][k]) = make_float2(xr[k], xr[k + 1]);
+        *reinterpret_cast<float2*>(&T.im[lane][k]) = make_float2(xi[k], xi[k + 1]);
+      }
+    }
+  }
+  if (!done) {
     __syncwarp();  // every lane has read its row
 #pragma unroll
     for (int k = 0; k < 32; ++k) {

@@ -2009,7 +2009,7 @@ int ps2_coherence_backward(ps2_ctx* c, const float* d_ph, const float* d_K, cons
     cb.wgrad = c->ad_win.p;
     cb.ab_partial = c->ad_part.as<double>();
     launched = cap;
-    CK(launch_clap_bwd(cb, fp64, c->twf, c->twd, &launched, st));
+    CK(launch_clap_bwd(cb, fp64, c->twd, &launched, st));
     // window-input gradients back onto the grid: the overlap gather is the
     // adjoint of the window extraction
     CK(launch_overlap(overlap_args(c, c->ad_win.p, c->ad_filt.p), fp64, st));

@@ -2865,21 +2865,19 @@ static int clap_bwd_blocks(int sm_count) {
 // Resident blocks of k_clap_bwd on the whole device (the size of the
 // alpha/beta partial array); 0 on error.
 int clap_bwd_max_blocks(int sm_count, bool fp64) {
-  return fp64 ? clap_bwd_blocks<double>(sm_count) : clap_bwd_blocks<float>(sm_count);
+  return fp64 ? clap_bwd_blocks<double>(sm_count) : clap_bwd_f32_max_blocks(sm_count);
 }
 
 // Launches at most *blocks_out blocks (the partial array's capacity) and
 // returns the number launched (0 when there are no windows).
-cudaError_t launch_clap_bwd(const ClapBwdArgs& b, bool fp64, const Twiddles32f& tf, const Twiddles32d& td,
-                            int* blocks_out, cudaStream_t st) {
+cudaError_t launch_clap_bwd(const ClapBwdArgs& b, bool fp64, const Twiddles32d& td, int* blocks_out,
+                            cudaStream_t st) {
   const int64_t ntask = static_cast<int64_t>(b.f.nwi) * b.f.nwj * (b.f.Mp / 4);
   const int64_t blocks = std::min<int64_t>(ntask, static_cast<int64_t>(*blocks_out));
   *blocks_out = static_cast<int>(std::max<int64_t>(blocks, 0));
   if (blocks <= 0) return cudaSuccess;
-  if (fp64)
-    k_clap_bwd<double><<<static_cast<unsigned>(blocks), 128, clap_bwd_smem<double>(), st>>>(b, td);
-  else
-    k_clap_bwd<float><<<static_cast<unsigned>(blocks), 128, clap_bwd_smem<float>(), st>>>(b, tf);
+  if (!fp64) return launch_clap_bwd_f32(b, static_cast<int>(blocks), st);
+  k_clap_bwd<double><<<static_cast<unsigned>(blocks), 128, clap_bwd_smem<double>(), st>>>(b, td);
   return cudaGetLastError();
 }
 
@@ -3114,7 +3112,6 @@ cudaError_t kernel_attributes_once(size_t dynamic_smem) {
         r == cudaSuccess ? opt_in_smem(k_s3_fit, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<float>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_topofit_near_max<double>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_clap_bwd<float>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap_bwd<double>, optin) : r,
     };
     cudaError_t first = cudaSuccess;

@@ -264,8 +264,10 @@ cudaError_t launch_coh(const CohArgs& a, int which /*0 fwd, 1 coherence bwd, 2 b
                        int sm_count, cudaStream_t st);
 cudaError_t launch_cell_sum(const CohArgs& a, const int32_t* cell_start, int64_t G, void* out, bool fp64,
                             int sm_count, cudaStream_t st);
-cudaError_t launch_clap_bwd(const ClapBwdArgs& b, bool fp64, const Twiddles32f& tf, const Twiddles32d& td,
-                            int* blocks_out, cudaStream_t st);
+cudaError_t launch_clap_bwd(const ClapBwdArgs& b, bool fp64, const Twiddles32d& td, int* blocks_out,
+                            cudaStream_t st);
+cudaError_t launch_clap_bwd_f32(const ClapBwdArgs& b, int blocks, cudaStream_t st);
+int clap_bwd_f32_max_blocks(int sm_count);
 int clap_bwd_max_blocks(int sm_count, bool fp64);
 cudaError_t launch_gather_widen(const float* src, double* dst, const int32_t* perm, int64_t n, cudaStream_t st);
 // dst[perm[s]] = double(src[s]) for an f32 vector, or 0.0 / 1.0 for a u8 flag vector (flags)
