@@ -1542,6 +1542,11 @@ int ps2_topofit_near_max(const void* cpxphase, const void* bperp, int32_t row_in
   a.C = dcc.as<double>();
   a.coh = dh.as<double>();
   a.residual = residual ? dr.as<float2>() : nullptr;
+  DevBuf dt;
+  if (const size_t b = topofit_near_max_table(fp64, row_inv != 0, n, a.M, n_half)) {
+    CK(dt.alloc(b));
+    a.table = dt.p;
+  }
   CK(launch_topofit_near_max(a, fp64, sc.sm, sc.st));
   CK(cudaMemcpyAsync(K, dk.p, sizeof(double) * n, cudaMemcpyDeviceToHost, sc.st));
   CK(cudaMemcpyAsync(C, dcc.p, sizeof(double) * n, cudaMemcpyDeviceToHost, sc.st));

@@ -300,7 +300,10 @@ struct NearMaxArgs {
   double* C;
   double* coh;
   float2* residual;  // complex64 [n, M] or NULL
+  void* table;       // complex [M][2 n_half + 1] work space, or NULL: trial phasors of a shared bp
 };
+// bytes of the table, 0 where rows evaluate their own phasors
+size_t topofit_near_max_table(bool fp64, bool row_inv, int64_t n, int M, int n_half);
 size_t topofit_near_max_smem(bool fp64, int M, int n_half);
 cudaError_t launch_topofit_near_max(const NearMaxArgs& a, bool fp64, int sm_count, cudaStream_t st);
 // histogram_with_centers (pystamps/kernels/accelerated.py:235-265)

@@ -86,3 +86,23 @@ def test_random_histogram_edges(S, oracle, m, n_trial_wraps, n_rand):
     b, bm = oracle.random_hist(bp, n_trial_wraps, n_rand=n_rand)
     np.testing.assert_array_equal(a, b)
     assert am == bm and a.sum() == n_rand
+
+
+# rows and table sizes either side of the rule for shared phasors: the general
+# path (a baseline matrix with equal rows) evaluates the same expressions
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("n,m,n_trial_wraps", [(1, 7, 1.0), (63, 30, 5.0), (64, 30, 5.0), (300, 1, 0.0), (300, 33, 4.0),
+                                               (70, 131, 500.0), (70, 132, 500.0)])
+def test_shared_baselines_give_the_general_path(cuda_lib, dtype, n, m, n_trial_wraps):
+    from pystamps_b200 import kernels as K
+
+    rng = np.random.default_rng(n + m)
+    z = np.exp(1j * rng.uniform(-math.pi, math.pi, (n, m))).astype(dtype)
+    z[::5, m // 2] = 0  # rows with a dropped column, whose own range may differ
+    z[n // 2] = 0
+    bp = rng.uniform(-300, 300, m).astype(z.real.dtype)
+    for b in (bp, np.full_like(bp, 25.0)):
+        one = K.run_stage2_topofit_row_invariant_kernel(z, b, n_trial_wraps)
+        gen = K._near_max(z, np.tile(b, (n, 1)), False, n_trial_wraps, K.NEAR_MAX_COH_TOL, dtype == np.complex64)
+        for x, y in zip(one, gen):
+            np.testing.assert_array_equal(x, y)
