@@ -33,6 +33,27 @@ def test_clap_window_sizes(cuda_lib, S, oracle, n_win, m, alpha):
     assert np.abs(out - ref).max() <= 64 * np.finfo(np.float32).eps * np.abs(ref).max()
 
 
+# warps a block (0: the rule), window stack or window blocks: every form the same bits
+@pytest.mark.parametrize("n_win", [8, 16, 24, 32])
+@pytest.mark.parametrize("m", [3, 8, 41])
+def test_clap_forms_give_the_same_bits(S, n_win, m):
+    from pystamps_b200 import synth
+
+    prep = S.prepare_patch(synth.make_patch(3000, m, 40, 41, seed=360 + m, n_rand=1000), nr=np.ones(100))
+    with S.Stage2Context() as c:
+        c.load(dataclasses.replace(prep, clap_window=n_win))
+        out = []
+        for warps in (0, 4, 8):
+            for form in (0, 1):
+                c.launch_shapes([0, warps, 0, 0, form])
+                c.reset()
+                c.iterate(2)
+                out.append(c.download(["ph_grid", "ph_patch", "K_ps", "coh_ps"]))
+    for o in out[1:]:
+        for k in o:
+            np.testing.assert_array_equal(o[k], out[0][k])
+
+
 @pytest.mark.parametrize("m", [3, 4, 7, 10])
 @pytest.mark.parametrize("slc_osf", [1, 2])
 def test_stage3_patches_at_even_and_odd_strides(cuda_lib, oracle, m, slc_osf):
