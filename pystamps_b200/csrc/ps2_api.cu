@@ -242,11 +242,10 @@ void gauss7(double* g, double* sum) {
   if (sum) *sum = s;
 }
 
-void twiddles(Twiddles32f* tf, Twiddles32d* td) {
+void twiddles(Twiddles32d* td) {
   for (int k = 0; k < 16; ++k) {
     const double a = -2.0 * M_PI * k / 32.0;
     td->w[k] = make_double2(std::cos(a), std::sin(a));
-    tf->w[k] = make_float2(static_cast<float>(std::cos(a)), static_cast<float>(std::sin(a)));
   }
 }
 
@@ -314,7 +313,6 @@ struct ps2_ctx {
   int64_t max_iter = 25;
   double cutoff0 = 0.01, dbin = 0.01;
   double g7[7], g7sum = 0.0;
-  Twiddles32f twf;
   Twiddles32d twd;
   DevBuf ph_nm, bp, amp, perm, cell_start, cell_of, w0, K[2], w, coh, C, nopt, grid, win, wpart, filt, low_pass, wscaled,
       taps, lut, nr0, nr_scaled, state, stats, hist, n_invalid, rms_partial, ph_res, scratch, stage;
@@ -706,7 +704,7 @@ int ps2_create(ps2_ctx** out, int device) {
     delete c;
     return set_err(PS2_ERR_CUDA, "ps2_create: %s", cudaGetErrorString(e));
   }
-  twiddles(&c->twf, &c->twd);
+  twiddles(&c->twd);
   gauss7(c->g7, &c->g7sum);
   coh_bin_rule(&c->cutoff0, &c->dbin);
   *out = c;
@@ -1645,9 +1643,8 @@ int ps2_clap_filter_grid(const float* ph_grid, int64_t n_i, int64_t n_j, int64_t
   a.wscaled = wsd.as<double>();
   gauss7(a.g7, nullptr);
   a.win_out = win.p;
-  Twiddles32f tf;
   Twiddles32d td;
-  twiddles(&tf, &td);
+  twiddles(&td);
   if (W > 0) {
     CK(launch_clap(a, false, td, sc.sm, sc.st));
     OverlapArgs o{};
@@ -1848,9 +1845,8 @@ int ps2_clap_filter_grid_noalloc(const float* d_ph_grid, int64_t n_i, int64_t n_
     a.wscaled = wsd;
     gauss7(a.g7, nullptr);
     a.win_out = win;
-    Twiddles32f tf;
     Twiddles32d td;
-    twiddles(&tf, &td);
+    twiddles(&td);
     CK(launch_clap(a, false, td, sms, st));
     OverlapArgs o{};
     o.win_out = win;
@@ -2372,9 +2368,6 @@ int ps3_reestimate(const ps3_reestimate_desc* d, ps3_reestimate_out* o, int devi
   CK(K2.alloc(sizeof(double) * n));
   CK(C2.alloc(sizeof(double) * n));
   CK(coh2.alloc(sizeof(double) * n));
-  Twiddles32f tf;
-  Twiddles32d td;
-  twiddles(&tf, &td);
   S3ClapArgs ca{};
   ca.grid = grid.as<float2>();
   ca.grid_cols = static_cast<int>(d->grid_cols);
@@ -2390,7 +2383,7 @@ int ps3_reestimate(const ps3_reestimate_desc* d, ps3_reestimate_out* o, int devi
   ca.low_pass = lp.as<double>();
   gauss7(ca.g7, nullptr);
   ca.job_out = jout.as<float2>();
-  ca.quarter_cos = tf.w[8].x;
+  ca.quarter_cos = static_cast<float>(std::cos(-2.0 * M_PI * 8 / 32.0));
   CK(launch_s3_clap(ca, sc.sm, st));
   S3FitArgs fa{};
   fa.ph = ph.as<float2>();
@@ -2505,7 +2498,7 @@ int ps2_stage3_reestimate(ps2_ctx* c, const int64_t* sel, int64_t n_sel, const i
   ca.low_pass = c->low_pass.as<double>();
   gauss7(ca.g7, nullptr);
   ca.job_out = jout.as<float2>();
-  ca.quarter_cos = c->twf.w[8].x;
+  ca.quarter_cos = static_cast<float>(std::cos(-2.0 * M_PI * 8 / 32.0));
   CK(launch_s3_clap(ca, c->sm_count, st));
   S3FitArgs fa{};
   fa.ph = c->ph_nm.as<float2>();

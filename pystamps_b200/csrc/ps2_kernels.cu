@@ -1,16 +1,18 @@
 // Stage-2 gamma-estimation kernels for B200 (sm_100a).
 //
 // One iteration of the reference loop (crates/pystamps-core/src/native_stage2.rs:261-406)
-// is five launches on one stream:
-//   k_bin       fill_phase_weight + accumulate_grid (:629-657, :722-740), fused,
-//               as a sort-by-cell sequential segmented reduction (no float atomics)
-//   k_clap      clap_filter_one_ifg per (window, ifg) (:823-916): 32x32 FFT in
-//               registers + shared memory, |H| smoothing, median, filter, IFFT
-//   k_overlap   the pyramid-weighted overlap-add (:904-915) as a gather in the
-//               reference's window order (deterministic)
-//   k_topofit   extract_patch_phase + fit_stage2_rows + topofit_row + refine_candidate
-//               (:1186-1303): one warp per PS, trial sweep by phasor recurrence
-//   k_finalize  rms_difference, stop rule, P-square weighting table (:307-381, :1538-1783)
+// is six launches on one stream; the FP32 CLAP and topofit kernels are in
+// clap_f32.cu and topofit_f32.cu, the others here:
+//   k_iter_begin   state of the last iteration kept, P-square weights (:1674-1682)
+//   k_bin          fill_phase_weight + accumulate_grid (:629-657, :722-740), fused,
+//                  as a sort-by-cell sequential segmented reduction (no float atomics)
+//   k_clap         clap_filter_one_ifg per (window, ifg) (:823-916): 32x32 FFT in
+//                  registers + shared memory, |H| smoothing, median, filter, IFFT
+//   k_overlap      the pyramid-weighted overlap-add (:904-915) as a gather in the
+//                  reference's window order (deterministic), and the unit patch phase
+//   k_topofit_f64  extract_patch_phase + fit_stage2_rows + topofit_row +
+//                  refine_candidate (:1186-1303)
+//   k_finalize     rms_difference, stop rule, P-square weighting table (:307-381, :1538-1783)
 #include <math.h>
 #include <stdint.h>
 
@@ -31,8 +33,6 @@ struct CT;
 template <>
 struct CT<float> {
   using C = float2;
-  using Tw = Twiddles32f;
-  using U = uint32_t;
 };
 template <>
 struct CT<double> {
@@ -271,23 +271,11 @@ template <>
 struct ClapShape<4> {
   static constexpr int kPad = 8;
 };
-__device__ __forceinline__ uint32_t to_bits(float v) { return __float_as_uint(v); }
 __device__ __forceinline__ unsigned long long to_bits(double v) {
   return static_cast<unsigned long long>(__double_as_longlong(v));
 }
-__device__ __forceinline__ float from_bits(uint32_t u) { return __uint_as_float(u); }
 __device__ __forceinline__ double from_bits(unsigned long long u) {
   return __longlong_as_double(static_cast<long long>(u));
-}
-__device__ __forceinline__ uint32_t warp_min_u(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = min(v, __shfl_xor_sync(kFull, v, o));
-  return v;
-}
-__device__ __forceinline__ uint32_t warp_max_u(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = max(v, __shfl_xor_sync(kFull, v, o));
-  return v;
 }
 __device__ __forceinline__ unsigned long long warp_min_u(unsigned long long v) {
 #pragma unroll

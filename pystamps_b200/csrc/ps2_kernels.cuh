@@ -7,9 +7,6 @@
 namespace ps2 {
 
 // e^{-2 pi i k / 32}, k = 0..15, computed on the host in double precision.
-struct Twiddles32f {
-  float2 w[16];
-};
 struct Twiddles32d {
   double2 w[16];
 };
@@ -149,7 +146,7 @@ struct S3ClapArgs {
   const double* low_pass;  // [32 * 32]
   double g7[7];
   float2* job_out;         // [n_jobs, M] filtered value at the PS cell
-  float quarter_cos;       // cos(pi / 2) as the twiddle tables round it (6e-17)
+  float quarter_cos;       // cos(pi / 2) as the host rounds it (6e-17)
 };
 
 struct S3FitArgs {
