@@ -307,7 +307,8 @@ __global__ void __launch_bounds__(256, 2) k_batch_clap(BatchArgs b) {
 // A block's four patches of one job (PS cell): interferograms 4 g .. 4 g + 3. Four
 // blocks an SM (57 KB and 128 registers each), sixteen warps as with eight a block,
 // and at most three idle warps at the end of the interferograms. 16,384 cells x 60
-// ifg: 10.9 -> 6.7 ms, with the window kernel's passes.
+// ifg: 10.9 -> 6.7 ms, with the window kernel's passes, inlined here (no spills at 128
+// registers; 7.3 ms with the transform out of line).
 struct S3Smem {
   ClapTileF<8> tiles[4];
   float lp[1024];
@@ -321,7 +322,7 @@ template <typename Tile>
 __device__ __forceinline__ float2 s3_patch_point(Tile& T, const int lane, const S3ClapArgs& a, const S3Smem& m,
                                                  const float (&g)[4], const int bi, const int bj) {
 #pragma unroll 1
-  for (int p = kForward1; p <= kForward2; ++p) fft_row<32>(T, lane, p, nullptr, 0, 0, 32);
+  for (int p = kForward1; p <= kForward2; ++p) fft_row_inline<32, 1>(T, lane, p, nullptr, 0, 0, 32);
   float o[32];
   smooth_tile(T, lane, g, o);
   float v0, v1;

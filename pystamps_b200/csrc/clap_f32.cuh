@@ -69,9 +69,9 @@ enum FftPass : int {
 // kInverse2 the lane's result times its pyramid weights wt[l] (l < nw) goes back to
 // its row.
 // FORM 0: all four passes; 1: the forward ones (adjoint's window); 2: the plain ones.
-template <int NZ, int FORM = 0, typename Tile>
-__device__ __noinline__ void fft_row(Tile& T, const int lane, const int p, const float* wt, const int rs, const int cs,
-                                     const int nw) {
+template <int NZ, int FORM, typename Tile>
+__device__ __forceinline__ void fft_row_inline(Tile& T, const int lane, const int p, const float* wt, const int rs,
+                                               const int cs, const int nw) {
   float2 ar[16], ai[16];  // points 2 m and 2 m + 1 at the bit reversal of m
   auto at = [](int m) { return ((m & 1) << 3) | ((m & 2) << 1) | ((m & 4) >> 1) | ((m & 8) >> 3); };
   bool done = false;
@@ -224,6 +224,14 @@ __device__ __noinline__ void fft_row(Tile& T, const int lane, const int p, const
     }
   }
   __syncwarp();
+}
+
+// The same out of line: the window kernels keep more registers live around it and
+// are faster so (256 x 256 cells x 60 ifg: 1258 against 1335 us an iteration).
+template <int NZ, int FORM = 0, typename Tile>
+__device__ __noinline__ void fft_row(Tile& T, const int lane, const int p, const float* wt, const int rs, const int cs,
+                                     const int nw) {
+  fft_row_inline<NZ, FORM>(T, lane, p, wt, rs, cs, nw);
 }
 
 // The 7-tap smoothing of 32 values along an axis of the fftshifted spectrum: in
