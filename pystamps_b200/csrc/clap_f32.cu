@@ -652,16 +652,15 @@ cudaError_t launch_nw(const ClapArgs& a, int sm_count, cudaStream_t st) {
 int64_t batch_clap_groups(int Mp) { return groups_f<8>(Mp); }
 
 // Warps a block unless the caller says: 4 where blocks of 8 would leave half a block
-// to the padding (Mp mod 8 = 4), where they would not fill the device once, and for
-// window blocks, whose serial windows want more blocks in flight; else 8, whose
-// sixteen warps an SM hide more than the twelve. us an iteration with 4 | 8:
-// 9 ifg 200 x 200 cells 232 | 261, 60 ifg 256 x 256 1254 | 1271, 30 ifg 30 x 30
-// 100 | 105, window blocks 150 ifg 256 x 256 2995 | 3088; 150 ifg 256 x 256 2934 | 2812.
+// to the padding (Mp mod 8 = 4) or would not fill the device once; else 8, whose
+// sixteen warps an SM hide more than the twelve. us an iteration with 4 | 8: 9 ifg
+// 200 x 200 cells 219 | 246, 60 ifg 256 x 256 1193 | 1204, 30 ifg 30 x 30 98 | 100;
+// 150 ifg 256 x 256 2778 | 2620.
 cudaError_t launch_clap_f32(const ClapArgs& a, int sm_count, cudaStream_t st) {
   int nw = a.nw_block;
   if (nw != 4 && nw != 8) {
     const int64_t windows = a.w_n > 0 ? a.w_n : static_cast<int64_t>(a.nwi) * a.nwj;
-    nw = a.part || a.Mp % 8 == 4 || windows * groups_f<8>(a.Mp) <= static_cast<int64_t>(sm_count) * 2 ? 4 : 8;
+    nw = a.Mp % 8 == 4 || windows * groups_f<8>(a.Mp) <= static_cast<int64_t>(sm_count) * 2 ? 4 : 8;
   }
   return nw == 4 ? launch_nw<4>(a, sm_count, st) : launch_nw<8>(a, sm_count, st);
 }

@@ -74,9 +74,7 @@ __device__ __forceinline__ void fft_row_inline(Tile& T, const int lane, const in
                                                const int cs, const int nw) {
   float2 ar[16], ai[16];  // points 2 m and 2 m + 1 at the bit reversal of m
   auto at = [](int m) { return ((m & 1) << 3) | ((m & 2) << 1) | ((m & 4) >> 1) | ((m & 8) >> 3); };
-  bool done = false;
   if (p == kForward1) {
-    done = true;
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
       const int j = at(m);
@@ -86,31 +84,19 @@ __device__ __forceinline__ void fft_row_inline(Tile& T, const int lane, const in
         ai[j] = *reinterpret_cast<const float2*>(&T.im[lane][2 * m]);
       }
     }
-  }
-  if constexpr (FORM == 0) {
-    if (p == kInverse1) {
-      done = true;
+  } else if (FORM != 1 && p == (FORM == 0 ? kInverse1 : kInverse1Plain)) {
 #pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const int j = at(m);
+    for (int m = 0; m < 16; ++m) {
+      const int j = at(m);
+      ar[j] = *reinterpret_cast<const float2*>(&T.im[lane][2 * m]);
+      ai[j] = *reinterpret_cast<const float2*>(&T.re[lane][2 * m]);
+      if constexpr (FORM == 0) {
         const float2 g = *reinterpret_cast<const float2*>(&T.hs[lane][2 * m]);
-        ar[j] = __fmul2_rn(*reinterpret_cast<const float2*>(&T.im[lane][2 * m]), g);
-        ai[j] = __fmul2_rn(*reinterpret_cast<const float2*>(&T.re[lane][2 * m]), g);
+        ar[j] = __fmul2_rn(ar[j], g);
+        ai[j] = __fmul2_rn(ai[j], g);
       }
     }
-  }
-  if constexpr (FORM == 2) {
-    if (p == kInverse1Plain) {
-      done = true;
-#pragma unroll
-      for (int m = 0; m < 16; ++m) {
-        const int j = at(m);
-        ar[j] = *reinterpret_cast<const float2*>(&T.im[lane][2 * m]);
-        ai[j] = *reinterpret_cast<const float2*>(&T.re[lane][2 * m]);
-      }
-    }
-  }
-  if (!done) {
+  } else {
 #pragma unroll
     for (int m = 0; m < 16; ++m) {
       const int j = at(m);
@@ -165,10 +151,8 @@ __device__ __forceinline__ void fft_row_inline(Tile& T, const int lane, const in
     xr[k + 16] = __fsub_rn(ur, tr);
     xi[k + 16] = __fsub_rn(ui, tj);
   }
-  done = false;
-  if constexpr (FORM != 2) {
-    if (p == kForward2) {
-      done = true;
+  if (FORM != 2 && p == kForward2) {
+    if constexpr (FORM != 2) {
       uint32_t far = 0;
 #pragma unroll
       for (int k = 0; k < 32; k += 2) {
@@ -187,33 +171,24 @@ __device__ __forceinline__ void fft_row_inline(Tile& T, const int lane, const in
           T.hs[k][lane] = sqrtf(__fmaf_rn(T.re[lane][k], T.re[lane][k], __fmul_rn(T.im[lane][k], T.im[lane][k])));
       }
     }
-  }
-  if constexpr (FORM == 0) {
-    if (p == kInverse2) {
-      done = true;
-      if (lane < nw) {
-        const bool row_zero = lane < rs;
+  } else if (FORM == 0 && p == kInverse2) {
+    if (lane < nw) {
+      const bool row_zero = lane < rs;
 #pragma unroll
-        for (int l = 0; l < NZ; l += 2) {
-          const float2 wv = make_float2((row_zero || l < cs || l >= nw) ? 0.f : wt[l],
-                                        (row_zero || l + 1 < cs || l + 1 >= nw) ? 0.f : wt[l + 1]);
-          *reinterpret_cast<float2*>(&T.re[lane][l]) = __fmul2_rn(make_float2(xr[l], xr[l + 1]), wv);
-          *reinterpret_cast<float2*>(&T.im[lane][l]) = __fmul2_rn(make_float2(xi[l], xi[l + 1]), wv);
-        }
+      for (int l = 0; l < NZ; l += 2) {
+        const float2 wv = make_float2((row_zero || l < cs || l >= nw) ? 0.f : wt[l],
+                                      (row_zero || l + 1 < cs || l + 1 >= nw) ? 0.f : wt[l + 1]);
+        *reinterpret_cast<float2*>(&T.re[lane][l]) = __fmul2_rn(make_float2(xr[l], xr[l + 1]), wv);
+        *reinterpret_cast<float2*>(&T.im[lane][l]) = __fmul2_rn(make_float2(xi[l], xi[l + 1]), wv);
       }
     }
-  }
-  if constexpr (FORM == 2) {
-    if (p == kForward2Plain || p == kInverse2Plain) {
-      done = true;
+  } else if (FORM == 2 && (p == kForward2Plain || p == kInverse2Plain)) {
 #pragma unroll
-      for (int k = 0; k < 32; k += 2) {
-        *reinterpret_cast<float2*>(&T.re[lane][k]) = make_float2(xr[k], xr[k + 1]);
-        *reinterpret_cast<float2*>(&T.im[lane][k]) = make_float2(xi[k], xi[k + 1]);
-      }
+    for (int k = 0; k < 32; k += 2) {
+      *reinterpret_cast<float2*>(&T.re[lane][k]) = make_float2(xr[k], xr[k + 1]);
+      *reinterpret_cast<float2*>(&T.im[lane][k]) = make_float2(xi[k], xi[k + 1]);
     }
-  }
-  if (!done) {
+  } else {
     __syncwarp();  // every lane has read its row
 #pragma unroll
     for (int k = 0; k < 32; ++k) {
@@ -227,7 +202,7 @@ __device__ __forceinline__ void fft_row_inline(Tile& T, const int lane, const in
 }
 
 // The same out of line: the window kernels keep more registers live around it and
-// are faster so (256 x 256 cells x 60 ifg: 1258 against 1335 us an iteration).
+// are faster so (256 x 256 cells x 60 ifg: 1194 against 1335 us an iteration).
 template <int NZ, int FORM = 0, typename Tile>
 __device__ __noinline__ void fft_row(Tile& T, const int lane, const int p, const float* wt, const int rs, const int cs,
                                      const int nw) {

@@ -1559,10 +1559,8 @@ cudaError_t launch_snr_weight(const TopoArgs& t, const float* amp, void* w_out, 
 }
 
 // ============================================== random-phase histogram ====
-// random_coherence_histogram / topofit_phase_row_coh (:1310-1512) in FP64:
-// one warp per random row, lanes over trials for the sweep (each lane sums its
-// trial over the columns in the reference's order), lanes over columns for the
-// refinement with the sums taken in column order by lane 0.
+// random_coherence_histogram / topofit_phase_row_coh (:1310-1512) in FP64; every
+// sum runs over the columns in the reference's order.
 // The trial phasors e^{-j theta_c m} of every (column, trial), theta_c =
 // (bp_c / range) * pi/4 (topofit_phase_row_coh, native_stage2.rs:1438-1470):
 // the same for every random row, so they are evaluated once, [m][T].
