@@ -881,7 +881,9 @@ cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32d& td, int
 
 // Overlap-add as a gather: cell (i, j) sums the windows that cover it, in the
 // reference's raster window order, in f64 (the reference accumulates in f64).
-template <typename R>
+// QUARTERS: n_win is a multiple of 4, windows n_win / 4 apart; 4 or 5 of them cover a
+// cell along an axis. Other sizes have n_inc = n_win / 4 rounded down and up to 10.
+template <typename R, bool QUARTERS>
 __device__ __forceinline__ void overlap_elem(const OverlapArgs& a, const int64_t idx) {
   using C = typename CT<R>::C;
   const C* __restrict__ win = static_cast<const C*>(a.win_out);
@@ -893,34 +895,51 @@ __device__ __forceinline__ void overlap_elem(const OverlapArgs& a, const int64_t
     const int i = static_cast<int>(cell / a.n_j), j = static_cast<int>(cell - static_cast<int64_t>(i) * a.n_j);
     double sx = 0.0, sy = 0.0;
     if (c < a.M && a.nwi > 0 && a.nwj > 0) {
-      const int a1 = max(0, i / a.n_inc - 4), b1 = min(a.nwi - 1, i / a.n_inc + 1);
-      const int a2 = max(0, j / a.n_inc - 4), b2 = min(a.nwj - 1, j / a.n_inc + 1);
-      // the (at most 6) candidate windows along j, their offsets and validity
-      int lj6[6];
-      bool okj[6];
+      const int qi = i / a.n_inc, qj = j / a.n_inc;
+      if constexpr (QUARTERS) {
+        // windows q - 3 .. q cover the cell, and the last one, clamped to the edge, may
+        const int a1 = max(0, qi - 3), b1 = min(a.nwi - 1, qi + 1);
+        const int a2 = max(0, qj - 3), b2 = min(a.nwj - 1, qj + 1);
+        // the (at most 5) candidate windows along j, their offsets and validity
+        int lj5[5];
+        bool ok5[5];
 #pragma unroll
-      for (int w = 0; w < 6; ++w) {
-        const int ix2 = a2 + w;
-        const int lj = j - min(ix2 * a.n_inc, a.n_j - nw);
-        okj[w] = ix2 <= b2 && lj >= 0 && lj < nw;
-        lj6[w] = lj;
-      }
-      for (int ix1 = a1; ix1 <= b1; ++ix1) {
-        const int i1 = min(ix1 * a.n_inc, a.n_i - nw);
-        const int li = i - i1;
-        if (li < 0 || li >= nw) continue;
-        // one row of covering windows: every load issued before the ordered sum
-        C v[6];
+        for (int w = 0; w < 5; ++w) {
+          const int ix2 = a2 + w;
+          const int lj = j - min(ix2 * a.n_inc, a.n_j - nw);
+          ok5[w] = ix2 <= b2 && lj >= 0;
+          lj5[w] = lj;
+        }
+        for (int ix1 = a1; ix1 <= b1; ++ix1) {
+          const int li = i - min(ix1 * a.n_inc, a.n_i - nw);
+          if (li < 0) continue;
+          // one row of covering windows: every load issued before the ordered sum
+          C v[5];
 #pragma unroll
-        for (int w = 0; w < 6; ++w)
-          v[w] = okj[w] ? win[((static_cast<int64_t>(ix1) * a.nwj + a2 + w) * nw2 + li * nw + lj6[w]) * a.Mp + c]
-                        : mk(R(0), R(0));
+          for (int w = 0; w < 5; ++w)
+            v[w] = ok5[w] ? win[((static_cast<int64_t>(ix1) * a.nwj + a2 + w) * nw2 + li * nw + lj5[w]) * a.Mp + c]
+                          : mk(R(0), R(0));
 #pragma unroll
-        for (int w = 0; w < 6; ++w)
-          if (okj[w]) {
-            sx += static_cast<double>(v[w].x);
-            sy += static_cast<double>(v[w].y);
+          for (int w = 0; w < 5; ++w)
+            if (ok5[w]) {
+              sx += static_cast<double>(v[w].x);
+              sy += static_cast<double>(v[w].y);
+            }
+        }
+      } else {
+        // window ix starts at min(ix n_inc, n - nw): those that cover a cell are a run,
+        // up to the last window (with others clamped alike) for an edge window's cells
+        const int a1 = i < nw ? 0 : (i - nw) / a.n_inc + 1, b1 = i >= a.n_i - nw ? a.nwi - 1 : min(a.nwi - 1, qi);
+        const int a2 = j < nw ? 0 : (j - nw) / a.n_inc + 1, b2 = j >= a.n_j - nw ? a.nwj - 1 : min(a.nwj - 1, qj);
+        for (int ix1 = a1; ix1 <= b1; ++ix1) {
+          const int li = i - min(ix1 * a.n_inc, a.n_i - nw);
+          for (int ix2 = a2; ix2 <= b2; ++ix2) {
+            const int lj = j - min(ix2 * a.n_inc, a.n_j - nw);
+            const C v = win[((static_cast<int64_t>(ix1) * a.nwj + ix2) * nw2 + li * nw + lj) * a.Mp + c];
+            sx += static_cast<double>(v.x);
+            sy += static_cast<double>(v.y);
           }
+        }
       }
     }
     C f = mk(static_cast<R>(sx), static_cast<R>(sy));
@@ -979,16 +998,22 @@ __device__ __forceinline__ void combine_elem(const OverlapArgs& a, const int64_t
 }
 
 template <typename R>
+__device__ __forceinline__ void overlap_any(const OverlapArgs& a, const int64_t idx) {
+  if (a.part)
+    combine_elem<R>(a, idx);
+  else if (a.n_win % 4 == 0)
+    overlap_elem<R, true>(a, idx);
+  else
+    overlap_elem<R, false>(a, idx);
+}
+
+template <typename R>
 __global__ void __launch_bounds__(256) k_overlap(OverlapArgs a) {
   const int64_t cells = a.cell_n > 0 ? a.cell_n : static_cast<int64_t>(a.n_i) * a.n_j;
   const int64_t total = cells * a.Mp, base = a.cell_lo * a.Mp;
   for (int64_t idx = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-       idx += static_cast<int64_t>(gridDim.x) * blockDim.x) {
-    if (a.part)
-      combine_elem<R>(a, base + idx);
-    else
-      overlap_elem<R>(a, base + idx);
-  }
+       idx += static_cast<int64_t>(gridDim.x) * blockDim.x)
+    overlap_any<R>(a, base + idx);
 }
 
 cudaError_t launch_overlap(const OverlapArgs& a, bool fp64, cudaStream_t st) {
@@ -2362,10 +2387,7 @@ __global__ void __launch_bounds__(256) k_batch_overlap(BatchArgs b) {
        u += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int p = find_patch(b.ov_prefix, b.P, u);
     if (!b.active[p]) continue;
-    if (b.patch[p].ov.part)
-      combine_elem<float>(b.patch[p].ov, u - b.ov_prefix[p]);
-    else
-      overlap_elem<float>(b.patch[p].ov, u - b.ov_prefix[p]);
+    overlap_any<float>(b.patch[p].ov, u - b.ov_prefix[p]);
   }
 }
 
