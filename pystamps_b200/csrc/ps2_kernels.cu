@@ -1047,7 +1047,7 @@ __host__ __device__ inline int f64_stride(int M) {
   const int mpad = (M + kF64Lanes - 1) / kF64Lanes * kF64Lanes;
   return (mpad / 8) % 2 ? mpad : mpad + 8;
 }
-// z, rotation and phasor per column: 48 bytes, 227 KB hold 7 warps at M = 150
+// z, rotation and phasor per column: 48 bytes; 58 KB a block at M = 150, six warps an SM
 static size_t topofit_f64_smem(int M) {
   return static_cast<size_t>(kF64Warps) * kF64Ps * f64_stride(M) * 3 * sizeof(double2);
 }
@@ -1078,7 +1078,7 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
   __shared__ int sh_hist[kCohBins];
   __shared__ double sh_rms[kF64Warps];
   __shared__ int sh_inv[kF64Warps];
-  __shared__ double sh_row[kF64Warps][kF64Ps][4];  // per row: range, trial K, refined K, sums
+  __shared__ double sh_row[kF64Warps][kF64Ps][4];  // per row: range, largest |bp| then trial K, refined K, sums
   for (int i = tid; i < kCohBins; i += blockDim.x) sh_hist[i] = 0;
   __syncthreads();
   const float2* __restrict__ ph_nm = static_cast<const float2*>(a.ph_nm);
@@ -1133,7 +1133,10 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
       mx = warp_max(mx);
       double range = mx - mn;
       if (range == 0.0) range = 1.0;
-      if (lane == 0) sh_row[wib][q][0] = range;
+      if (lane == 0) {
+        sh_row[wib][q][0] = range;
+        sh_row[wib][q][1] = fmax(fabs(mn), fabs(mx));
+      }
     }
     __syncwarp();
     for (int idx = lane; idx < rows * mpad; idx += 32) {
@@ -1228,9 +1231,14 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
         top.t = ot;
       }
     }
-    // a chain's phasor is off by at most ~3e-16 a step, a sum by that times
-    // sum |z|, its square by 2 (sum |z|)^2 times that; (sum |z|)^2 <= M sum |z|^2
-    const double tol = 4.0e-15 * (a.n_half + 64) * a.M * zz;
+    // a chain's phasor is off by at most ~3e-16 a step, the direct sum's by the
+    // rounding of its argument theta m (2^-53 of it), a sum by that times sum |z|,
+    // its square by 2 (sum |z|)^2 times that; (sum |z|)^2 <= M sum |z|^2, and two
+    // squares are compared. theta is large where the baselines lie close together
+    // far from zero
+    const float th_max = static_cast<float>(sh_row[wib][g < rows ? g : 0][1]) /
+                         static_cast<float>(sh_row[wib][g < rows ? g : 0][0]);  // in units of pi / 4
+    const double tol = (4.0e-15 * (a.n_half + 64) + 4.0e-16 * th_max * a.n_half) * a.M * zz;
     const unsigned clear = __ballot_sync(kFull, top.best - top.second > tol);
     for (int q = 0; q < rows; ++q) {
       const int64_t s = s0 + q;
