@@ -1031,25 +1031,32 @@ cudaError_t launch_overlap(const OverlapArgs& a, bool fp64, cudaStream_t st) {
 
 // Plain FP64 topofit, the comparison path; it shares only the data layout with
 // the FP32 kernel. A direct sincos for every (trial, column) made it 77 % of an
-// FP64 iteration. A warp takes kF64Ps rows: their z and theta go to shared memory
+// FP64 iteration. A warp takes 32 / L rows: their z and theta go to shared memory
 // (lanes over columns, a row at a time); the trial sums of the rows run side by
-// side (8 lanes a row, lanes over columns) as phasor chains, trials +-m from one
+// side (L = 8 or 16 lanes a row, lanes over columns) as phasor chains, trials +-m from one
 // chain; each row's refinement is again the warp's, lanes over columns. The
 // chains only rank the trials: where the best one does not lead by more than
 // their rounding error, the row's trials are evaluated again by the direct sum
 // (every lane its trials, columns in order), so the trial chosen is the direct
 // sum's. 100,000 PS x 40 ifg x 121 trials: 1.73 -> 0.57 ms.
-constexpr int kF64Lanes = 8, kF64Ps = 32 / kF64Lanes, kF64Warps = 2, kF64W = 8;
+constexpr int kF64Warps = 2, kF64W = 8;
 
-// Row stride in columns: M padded to the lanes, an odd multiple of 8 so that the
-// four rows of a warp start in different banks.
-__host__ __device__ inline int f64_stride(int M) {
-  const int mpad = (M + kF64Lanes - 1) / kF64Lanes * kF64Lanes;
-  return (mpad / 8) % 2 ? mpad : mpad + 8;
+// Columns padded to the L lanes of a row.
+template <int L>
+__host__ __device__ inline int f64_mpad(int M) {
+  return (M + L - 1) / L * L;
 }
-// z, rotation and phasor per column: 48 bytes; 58 KB a block at M = 150, six warps an SM
+// Row stride in columns: an odd multiple of 8, so that the rows of a warp start in
+// different banks.
+template <int L>
+__host__ __device__ inline int f64_stride(int M) {
+  return (f64_mpad<L>(M) / 8) % 2 ? f64_mpad<L>(M) : f64_mpad<L>(M) + 8;
+}
+// z, rotation and phasor per column: 48 bytes; at M = 150 and 16 lanes a row 32 KB a
+// block, fourteen warps an SM
+template <int L>
 static size_t topofit_f64_smem(int M) {
-  return static_cast<size_t>(kF64Warps) * kF64Ps * f64_stride(M) * 3 * sizeof(double2);
+  return static_cast<size_t>(kF64Warps) * (32 / L) * f64_stride<L>(M) * 3 * sizeof(double2);
 }
 
 // Trial -> best |S|^2, its trial (the first on ties) and the largest |S|^2 among the others.
@@ -1067,18 +1074,19 @@ struct Top2 {
   }
 };
 
+template <int L>
 __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
+  constexpr int PS = 32 / L;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int tid = threadIdx.x, lane = tid & 31, wib = tid >> 5;
-  const int stride = f64_stride(a.M);
-  const int mpad = (a.M + kF64Lanes - 1) / kF64Lanes * kF64Lanes;
-  double2* zs0 = reinterpret_cast<double2*>(smem_raw) + static_cast<int64_t>(wib) * kF64Ps * stride * 3;
-  double2* rot0 = zs0 + kF64Ps * stride;
-  double2* ph0 = rot0 + kF64Ps * stride;
+  const int stride = f64_stride<L>(a.M), mpad = f64_mpad<L>(a.M);
+  double2* zs0 = reinterpret_cast<double2*>(smem_raw) + static_cast<int64_t>(wib) * PS * stride * 3;
+  double2* rot0 = zs0 + PS * stride;
+  double2* ph0 = rot0 + PS * stride;
   __shared__ int sh_hist[kCohBins];
   __shared__ double sh_rms[kF64Warps];
   __shared__ int sh_inv[kF64Warps];
-  __shared__ double sh_row[kF64Warps][kF64Ps][4];  // per row: range, largest |bp| then trial K, refined K, sums
+  __shared__ double sh_row[kF64Warps][PS][4];  // per row: range, largest |bp| then trial K, refined K, sums
   for (int i = tid; i < kCohBins; i += blockDim.x) sh_hist[i] = 0;
   __syncthreads();
   const float2* __restrict__ ph_nm = static_cast<const float2*>(a.ph_nm);
@@ -1096,9 +1104,9 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
   int inv_acc = 0;
   const int64_t gw = (static_cast<int64_t>(blockIdx.x) * blockDim.x + tid) >> 5;
   const int64_t nwarps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int g = lane / kF64Lanes, gl = lane % kF64Lanes;
-  for (int64_t s0 = gw * kF64Ps; s0 < a.N; s0 += nwarps * kF64Ps) {
-    const int rows = a.N - s0 < kF64Ps ? static_cast<int>(a.N - s0) : kF64Ps;
+  const int g = lane / L, gl = lane % L;
+  for (int64_t s0 = gw * PS; s0 < a.N; s0 += nwarps * PS) {
+    const int rows = a.N - s0 < PS ? static_cast<int>(a.N - s0) : PS;
     unsigned invalid_rows = 0;
     __syncwarp();
     // elementwise steps run over all elements of the rows, so that no lane idles at
@@ -1156,16 +1164,16 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
     double zz = 0.0, sx0 = 0.0, sy0 = 0.0;
     if (g < rows) {
       const double2* zs = zs0 + g * stride;
-      for (int c = gl; c < mpad; c += kF64Lanes) {
+      for (int c = gl; c < mpad; c += L) {
         const double2 z = zs[c];
         sx0 += z.x;
         sy0 += z.y;
         zz += z.x * z.x + z.y * z.y;
       }
     }
-    sx0 = group_sum<kF64Lanes>(sx0);
-    sy0 = group_sum<kF64Lanes>(sy0);
-    zz = group_sum<kF64Lanes>(zz);
+    sx0 = group_sum<L>(sx0);
+    sy0 = group_sum<L>(sy0);
+    zz = group_sum<L>(zz);
     if (gl == 0) top.add(sx0 * sx0 + sy0 * sy0, a.n_half);
     for (int m0 = 1; m0 <= a.n_half; m0 += kF64W) {
       double2 A[kF64W], B[kF64W];  // (sum x w.x, sum x w.y), (sum y w.x, sum y w.y)
@@ -1175,7 +1183,7 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
         const double2* zs = zs0 + g * stride;
         const double2* rot = rot0 + g * stride;
         double2* ph = ph0 + g * stride;
-        for (int c = gl; c < mpad; c += kF64Lanes) {
+        for (int c = gl; c < mpad; c += L) {
           const double2 z = zs[c], r = rot[c];
           double2 w = ph[c];
 #pragma unroll
@@ -1199,7 +1207,7 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
       }
       int base = 0;
 #pragma unroll
-      for (int o = kF64Lanes / 2, h = kF64W; o >= 1; o >>= 1, h >>= 1) {
+      for (int o = L / 2, h = kF64W; o >= 1; o >>= 1, h >>= 1) {
         const bool upper = (gl & o) != 0;
 #pragma unroll
         for (int i = 0; i < kF64W; ++i) {
@@ -1215,13 +1223,13 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
         if (upper) base += h;
       }
 #pragma unroll
-      for (int i = 0; i < 2 * kF64W / kF64Lanes; ++i) {
+      for (int i = 0; i < 2 * kF64W / L; ++i) {
         const int idx = base + i, m = m0 + (idx < kF64W ? idx : idx - kF64W);
         if (m <= a.n_half) top.add(S[i].x * S[i].x + S[i].y * S[i].y, idx < kF64W ? a.n_half + m : a.n_half - m);
       }
     }
 #pragma unroll
-    for (int o = kF64Lanes / 2; o > 0; o >>= 1) {
+    for (int o = L / 2; o > 0; o >>= 1) {
       const double ob = __shfl_xor_sync(kFull, top.best, o), os = __shfl_xor_sync(kFull, top.second, o);
       const int ot = __shfl_xor_sync(kFull, top.t, o);
       const bool theirs = ob > top.best || (ob == top.best && ot < top.t);
@@ -1245,8 +1253,8 @@ __global__ void __launch_bounds__(32 * kF64Warps) k_topofit_f64(TopoArgs a) {
       const double2* zs = zs0 + q * stride;
       double2* rot = rot0 + q * stride;
       const double range = sh_row[wib][q][0];
-      int bt = __shfl_sync(kFull, top.t, q * kF64Lanes);
-      if (!((invalid_rows >> q) & 1u) && !((clear >> (q * kF64Lanes)) & 1u)) {
+      int bt = __shfl_sync(kFull, top.t, q * L);
+      if (!((invalid_rows >> q) & 1u) && !((clear >> (q * L)) & 1u)) {
         for (int c = lane; c < a.M; c += 32) {
           const double b = a.bp_row_inv ? static_cast<double>(a.bp[c]) : static_cast<double>(a.bp[s * M + c]);
           rot[c].x = (b / range) * qpi;
@@ -1416,16 +1424,27 @@ int64_t clap_part_elems(int nwi, int nwj, int n_win, int Mp) {
   return std::max<int64_t>(static_cast<int64_t>(clap_block_rows(nwi)) * clap_block_rows(nwj), 1) * box * box * Mp;
 }
 
+template <int L>
+static cudaError_t launch_topofit_f64(const TopoArgs& a, int grid_blocks, cudaStream_t st) {
+  const int64_t per_block = kF64Warps * (32 / L);
+  const int blocks = static_cast<int>(std::min<int64_t>((a.N + per_block - 1) / per_block, grid_blocks));
+  const size_t sm = topofit_f64_smem<L>(a.M);
+  cudaError_t e = kernel_attributes_once(sm);
+  if (e != cudaSuccess) return e;
+  k_topofit_f64<L><<<blocks, 32 * kF64Warps, sm, st>>>(a);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_topofit(const TopoArgs& a, bool fp64, int grid_blocks, cudaStream_t st) {
   if (a.N <= 0) return cudaSuccess;
   if (fp64) {
-    const int64_t need = (a.N + kF64Warps * kF64Ps - 1) / (kF64Warps * kF64Ps);
-    const int blocks = static_cast<int>(std::min<int64_t>(need, grid_blocks));
-    const size_t sm = topofit_f64_smem(a.M);
-    cudaError_t e = kernel_attributes_once(sm);
-    if (e != cudaSuccess) return e;
-    k_topofit_f64<<<blocks, 32 * kF64Warps, sm, st>>>(a);
-    return cudaGetLastError();
+    // 8 lanes a row spend the fewest instructions; 16 hold half the rows a warp, so
+    // twice the warps stay resident where the rows' columns fill the shared memory, and
+    // more run where there are few rows (up to 32 an SM). us with 16 | 8 lanes: 30,000
+    // rows x 121 trials, 40 ifg 208 | 153, 60 ifg 244 | 232, 100 ifg 349 | 362, 200 ifg
+    // 731 | 1118, 256 ifg and 9 trials 635 | 1068; 3,000 rows x 20 ifg x 41 20.5 | 24.1
+    const bool wide = a.M > 64 || a.N <= 2 * static_cast<int64_t>(grid_blocks);
+    return wide ? launch_topofit_f64<16>(a, grid_blocks, st) : launch_topofit_f64<8>(a, grid_blocks, st);
   }
   return launch_topofit_f32(a, grid_blocks, st);
 }
@@ -3171,7 +3190,8 @@ cudaError_t kernel_attributes_once(size_t dynamic_smem) {
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 24, false>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 0, true>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_clap<double, 4, 24, true>, optin) : r,
-        r == cudaSuccess ? opt_in_smem(k_topofit_f64, optin) : r,
+        r == cudaSuccess ? opt_in_smem(k_topofit_f64<8>, optin) : r,
+        r == cudaSuccess ? opt_in_smem(k_topofit_f64<16>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_random_hist<4>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_random_hist<8>, optin) : r,
         r == cudaSuccess ? opt_in_smem(k_s3_fit, optin) : r,

@@ -105,3 +105,12 @@ def test_tied_trials(cuda_lib, m, trials, n):
     assert ok.sum() > 0.9 * n
     np.testing.assert_allclose(near[ok], 0.0, atol=1e-10 * max(1.0, QPI * half))
     np.testing.assert_allclose(cohs[ok], 0.0, atol=1e-11)
+
+
+# 16 lanes take a row above 64 columns or in launches of few rows, 8 the others: 8-lane
+# launches at the edges of the lanes and trial blocks, and either side of the column rule
+@pytest.mark.parametrize("m,trials", [(7, 1), (8, 17), (9, 19), (31, 41), (33, 35), (64, 33), (65, 33)])
+def test_launches_of_many_rows(cuda_lib, m, trials):
+    from test_gpu_topofit_f64 import test_trial_and_refinement as check
+
+    check(cuda_lib, m, trials, 5003, False)
