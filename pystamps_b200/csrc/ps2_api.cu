@@ -896,11 +896,13 @@ int ps2_load_patch(ps2_ctx* c, const ps2_patch_desc* d) {
   CK(c->nr_scaled.alloc(sizeof(double) * PS2_COH_BINS));
   CK(c->state.alloc(sizeof(double) * 4));
   CK(c->stats.alloc(sizeof(double) * 8));
-  // a block may hold an earlier owner's data: what a download before the first
-  // iteration reads starts at zero
+  // a block may hold an earlier owner's data: what a download, an export or a stage-3
+  // call before the first iteration reads starts at zero
   CK(cudaMemsetAsync(c->C.p, 0, R * N, c->st));
   CK(cudaMemsetAsync(c->nopt.p, 0, N, c->st));
   CK(cudaMemsetAsync(c->stats.p, 0, sizeof(double) * 8, c->st));
+  CK(cudaMemsetAsync(c->grid.p, 0, Cz * G * c->Mp, c->st));
+  if (!c->psquare) CK(cudaMemsetAsync(c->ph_res.p, 0, R * N * M, c->st));
   CK(c->hist.alloc(sizeof(int32_t) * PS2_COH_BINS));
   CK(c->n_invalid.alloc(sizeof(int32_t)));
   c->topo_blocks = topofit_grid_blocks(c->sm_count, c->fp64);
