@@ -86,15 +86,18 @@ class DeviceCache {
     static DeviceCache* c = new DeviceCache();  // never destroyed: the driver may end before static objects do
     return *c;
   }
-  // Blocks are rounded up to 1/8 of their power of two (512 bytes at least), and
-  // a kept block serves requests down to 3/4 of its size: waste stays below a third.
+  // Blocks that may be kept are rounded up to a sixteenth of their size (512 bytes at
+  // least), and a kept block serves requests down to 3/4 of its size: waste stays
+  // below a third. Larger ones are allocated as they are asked for.
+  static size_t exact(size_t n) { return (n + 511) / 512 * 512; }
   static size_t rounded(size_t n) {
+    if (n > kMaxBlock) return exact(n);
     size_t g = 512;
     while (g * 16 <= n) g *= 2;
     return (n + g - 1) / g * g;
   }
   cudaError_t alloc(void** p, size_t* bytes, int* device) {
-    const size_t want = rounded(*bytes);
+    size_t want = rounded(*bytes);
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
@@ -119,6 +122,7 @@ class DeviceCache {
     if (e == cudaErrorMemoryAllocation && dev < kMaxDevices) {
       cudaGetLastError();
       give_back(dev);
+      want = exact(*bytes);
       e = cudaMalloc(p, want);
     }
     if (e == cudaSuccess) *bytes = want;
