@@ -52,7 +52,7 @@ extern "C" {
 #define PS2_ERR_OUT_OF_MEMORY (-5)
 
 #define PS2_PRECISION_FP32 0 /* FP32 compute, FP64 only in K refinement and weighting */
-#define PS2_PRECISION_FP64 1 /* plain FP64 everywhere (direct sincos, no recurrence) */
+#define PS2_PRECISION_FP64 1 /* plain FP64 everywhere; the trial is the direct sums' */
 
 #define PS2_COH_BINS 100
 
@@ -119,6 +119,13 @@ typedef struct ps2_outputs {
 int ps2_create(ps2_ctx** out, int device);
 void ps2_destroy(ps2_ctx* ctx);
 const char* ps2_last_error(void);
+/* Calls and destroyed contexts leave device memory and idle streams with the
+ * process for the next ones: up to 512 MiB and 16 streams a device, safe from
+ * several threads, handed back by themselves when an allocation of this library
+ * fails. ps2_release_kept hands them back to the driver now (for example before
+ * another allocator of the process needs the memory, or before a device reset);
+ * *bytes, unless NULL, receives the memory's size. What loaded contexts hold stays. */
+int ps2_release_kept(int64_t* bytes);
 /* Uploads and lays out one patch (cell-sorted rows). Copies the inputs; no
  * caller pointer is retained after return. */
 int ps2_load_patch(ps2_ctx* ctx, const ps2_patch_desc* desc);

@@ -39,6 +39,7 @@ EXPORTED = (
     "ps2_stage3_reestimate", "ps2_shard_bin", "ps2_shard_filter", "ps2_shard_fit", "ps2_shard_finalize",
     "ps2_prepare_phase", "ps2_prepare_bperp", "ps2_topofit_near_max", "ps2_histogram_with_centers",
     "ps2_export_state", "ps2_import_state", "ps2_step", "ps2_launch_shapes",
+    "ps2_release_kept",
 )
 
 
@@ -126,6 +127,14 @@ def check(rc: int) -> None:
     if rc != PS2_OK:
         msg = lib().ps2_last_error().decode(errors="replace")
         raise Stage2CudaError(rc, msg)
+
+
+def release_kept() -> int:
+    """Hand the device memory and streams kept between calls (at most 512 MiB and
+    16 streams a device) back to the driver; returns the bytes (ps2_release_kept)."""
+    n = ctypes.c_int64(0)
+    check(lib().ps2_release_kept(ctypes.byref(n)))
+    return n.value
 
 
 def ptr(a) -> int:

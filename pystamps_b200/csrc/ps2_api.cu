@@ -175,16 +175,32 @@ class DeviceCache {
     }
     cudaStreamDestroy(s);
   }
+  // Every device's kept blocks and streams back to the driver; the blocks' bytes.
+  size_t give_back_all() {
+    size_t bytes = 0;
+    for (int dev = 0; dev < kMaxDevices; ++dev) {
+      bytes += give_back(dev);
+      std::vector<cudaStream_t> idle;
+      {
+        std::lock_guard<std::mutex> g(mu_);
+        idle.swap(streams_[dev]);
+      }
+      for (cudaStream_t s : idle) cudaStreamDestroy(s);
+    }
+    return bytes;
+  }
 
  private:
-  void give_back(int dev) {
+  size_t give_back(int dev) {
     std::vector<std::pair<void*, size_t>> all;
+    size_t bytes = 0;
     {
       std::lock_guard<std::mutex> g(mu_);
       all.swap(blocks_[dev]);
-      held_[dev] = 0;
+      std::swap(bytes, held_[dev]);
     }
     for (auto& b : all) cudaFree(b.first);
+    return bytes;
   }
   std::mutex mu_;
   std::vector<std::pair<void*, size_t>> blocks_[kMaxDevices];
@@ -691,6 +707,12 @@ size_t state_bytes(ps2_ctx* c) {
 extern "C" {
 
 const char* ps2_last_error(void) { return g_err.c_str(); }
+
+int ps2_release_kept(int64_t* bytes) {
+  const size_t freed = DeviceCache::get().give_back_all();
+  if (bytes) *bytes = static_cast<int64_t>(freed);
+  return PS2_OK;
+}
 
 int ps2_create(ps2_ctx** out, int device) {
   if (!out) return set_err(PS2_ERR_INVALID_ARG, "ps2_create: out is NULL");
