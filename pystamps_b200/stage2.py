@@ -279,18 +279,21 @@ class Stage2Context:
         self.prepared: PreparedPatch | None = None
         self.precision = PRECISION_FP32
         self._keep = []
-        self._rows = self._rows_lease = None
+        self._results: dict[str, list] = {}
 
-    def _result_rows(self, count: int, n: int) -> list[np.ndarray]:
-        """`count` float64 vectors of length n for a download. Their memory is kept
-        by the context and used again once every vector handed out from it is gone
-        (fresh pages cost more to touch than the copy: 1.5 of 5 ms for 250,000 PS)."""
-        if self._rows is None or self._rows.size < count * n or self._rows_lease() is not None:
-            self._rows = np.empty(count * n, dtype=np.float64)
-        # the vectors' base is this view, not the memory's owner: it lives as long as any of them
-        lease = np.frombuffer(memoryview(self._rows), dtype=np.float64)
-        self._rows_lease = weakref.ref(lease)
-        return [lease[k * n:(k + 1) * n] for k in range(count)]
+    def _result_vector(self, key: str, n: int) -> np.ndarray:
+        """A float64 vector of length n for a download. The context keeps the memory of
+        the last two of each key and hands one out again once neither it nor a view of
+        it is left: a loop that drops a result after the next one arrives takes the two
+        in turn (fresh pages cost more to touch than the copy: 1.5 of 5 ms for 250,000
+        PS). Keys share no memory."""
+        kept = [e for e in self._results.get(key, ()) if e[0].size == n]
+        free = next((e for e in kept if e[1]() is None), None)
+        memory = np.empty(n, dtype=np.float64) if free is None else free[0]
+        # the result is a view whose base is no array: views of it refer to itself
+        vector = np.frombuffer(memoryview(memory), dtype=np.float64)
+        self._results[key] = [e for e in kept if e is not free][-1:] + [(memory, weakref.ref(vector))]
+        return vector
 
     def close(self) -> None:
         if self._ctx:
@@ -431,9 +434,6 @@ class Stage2Context:
         given = out or {}
         out = {}
         o = _lib.Outputs()
-        vectors = [k for k in ("K_ps", "C_ps", "coh_ps", "N_opt", "coh_ps_save") if k in want]
-        fresh = [k for k in vectors if given.get(k) is None]
-        rows = dict(zip(fresh, self._result_rows(len(fresh), n)))
         for k in ("K_ps", "C_ps", "coh_ps", "N_opt", "coh_ps_save"):
             if k in want:
                 g = given.get(k)
@@ -444,7 +444,7 @@ class Stage2Context:
                                          f"of length {n}")
                     out[k] = g
                 else:
-                    out[k] = rows[k]
+                    out[k] = self._result_vector(k, n)
                 setattr(o, k, ptr(out[k]))
         cdt, rdt = (np.complex128, np.float64) if fp64 else (np.complex64, np.float32)
         suffix = "_f64" if fp64 else ""
