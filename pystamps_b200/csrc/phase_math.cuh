@@ -53,12 +53,15 @@ __device__ __forceinline__ float atan2_poly(float y, float x) {
 }
 __device__ __forceinline__ float2 both(const float v) { return make_float2(v, v); }
 
-// Square roots of two values by one Newton step from the reciprocal square root
-// approximation: y ~ 1 / sqrt(q), s = q y, s + (q - s^2) y / 2 with the residual exact
-// in one FMA. Equal to sqrtf for every float in [2^-100, infinity) (all 1.9e9 bit
-// patterns compared); outside, callers take sqrtf itself. 5 instructions a value
-// against 25 for sqrtf, whose range checks branch value by value: magnitudes were
-// a fifth of a window's time.
+// Square roots by one step of Heron's iteration in the form Markstein gives it for
+// machines with a fused multiply-add ("Computation of elementary functions on the IBM
+// RISC System/6000 processor", IBM J. Res. Dev. 34, 1990): with y ~ 1 / sqrt(q) and
+// s = q y, s + (q - s^2) / (2 s) is taken as s + (q - s^2) (y / 2). An approximation
+// good to 2^-22 leaves an error of its square before the last rounding. The residual
+// is exact in one FMA: its last bit is no lower than that of s^2, 2^-146 for q >=
+// 2^-100, and FP32 goes to 2^-149. Equal to sqrtf for every float in [2^-100,
+// infinity) (tests/test_gpu_sqrt.py compares them all); other values take sqrtf itself.
+// sqrtf in its place made magnitudes a fifth of a window's time.
 constexpr uint32_t kSqrtLo = 0x0d800000u;                // 2^-100
 constexpr uint32_t kSqrtSpan = 0x7f800000u - kSqrtLo;  // up to infinity
 __device__ __forceinline__ float2 sqrt_newton2(const float2 q) {
