@@ -632,13 +632,17 @@ cudaError_t launch_form(const ClapArgs& a, const int64_t ntask, int sm_count, cu
   return cudaGetLastError();
 }
 
+// Windows, or window blocks where the partials are asked for, of a launch.
+int64_t units_f(const ClapArgs& a) {
+  if (a.w_n > 0) return a.w_n;
+  return a.part ? static_cast<int64_t>(clap_block_rows(a.nwi)) * clap_block_rows(a.nwj)
+                : static_cast<int64_t>(a.nwi) * a.nwj;
+}
+
 template <int NW>
 cudaError_t launch_nw(const ClapArgs& a, int sm_count, cudaStream_t st) {
   if (a.nwi <= 0 || a.nwj <= 0) return cudaSuccess;
-  const int64_t nunit = a.w_n > 0 ? a.w_n
-                        : a.part ? static_cast<int64_t>(clap_block_rows(a.nwi)) * clap_block_rows(a.nwj)
-                                 : static_cast<int64_t>(a.nwi) * a.nwj;
-  const int64_t ntask = nunit * groups_f<NW>(a.Mp);
+  const int64_t ntask = units_f(a) * groups_f<NW>(a.Mp);
   if (ntask <= 0) return cudaSuccess;
   if (a.n_win == 24)
     return a.part ? launch_form<NW, 24, true>(a, ntask, sm_count, st)
@@ -651,16 +655,26 @@ cudaError_t launch_nw(const ClapArgs& a, int sm_count, cudaStream_t st) {
 
 int64_t batch_clap_groups(int Mp) { return groups_f<8>(Mp); }
 
-// Warps a block unless the caller says: 4 where blocks of 8 would leave half a block
-// to the padding (Mp mod 8 = 4) or would not fill the device once; else 8, whose
-// sixteen warps an SM hide more than the twelve. us an iteration with 4 | 8: 9 ifg
-// 200 x 200 cells 219 | 246, 60 ifg 256 x 256 1193 | 1204, 30 ifg 30 x 30 98 | 100;
-// 150 ifg 256 x 256 2778 | 2620.
+// Warps a block unless the caller says. 8 (two blocks, sixteen warps an SM) hide more
+// than 4 (three blocks, twelve), and 4 finish a partly filled device sooner: 4 where
+// all their blocks fit at once, else 8 where those do, else by the padding: with Mp mod
+// 8 = 4 blocks of 8 idle 4 / (Mp + 4) of their warps, which costs more than 12 for 16
+// up to Mp = 60, and at any Mp where two rounds of blocks do or in window blocks, whose
+// few long tasks leave a longer tail. us with 4 | 8 warps, window stack: 200 x 200 cells
+// 12 ifg 123 | 155, 28 278 | 294, 60 567 | 565, 100 932 | 887, 148 1369 | 1318, 150
+// 1422 | 1328; 64 x 64 x 28 38.0 | 33.6; 40 x 40 cells 100 ifg 31.7 | 33.7, 116 38.5 |
+// 33.9, 148 42.0 | 44.5. Window blocks: 40 x 40 x 150 180 | 240; 128 x 128 x 132 531 |
+// 655, 76 385 | 372; 200 x 200 x 84 871 | 954.
 cudaError_t launch_clap_f32(const ClapArgs& a, int sm_count, cudaStream_t st) {
   int nw = a.nw_block;
   if (nw != 4 && nw != 8) {
-    const int64_t windows = a.w_n > 0 ? a.w_n : static_cast<int64_t>(a.nwi) * a.nwj;
-    nw = a.Mp % 8 == 4 || windows * groups_f<8>(a.Mp) <= static_cast<int64_t>(sm_count) * 2 ? 4 : 8;
+    const int64_t units = units_f(a), fours = units * groups_f<4>(a.Mp), once = static_cast<int64_t>(sm_count) * 3;
+    if (fours <= once)
+      nw = 4;
+    else if (!a.part && units * groups_f<8>(a.Mp) <= static_cast<int64_t>(sm_count) * 2)
+      nw = 8;
+    else
+      nw = a.Mp % 8 == 4 && (a.part || a.Mp <= 60 || fours <= 2 * once) ? 4 : 8;
   }
   return nw == 4 ? launch_nw<4>(a, sm_count, st) : launch_nw<8>(a, sm_count, st);
 }

@@ -82,3 +82,23 @@ def test_loop_forms(cuda_lib, n_win, precision):
             np.testing.assert_array_equal(out[0][k], out[1][k])
     else:  # the two forms add a cell's windows in FP64 in different orders
         assert np.abs(out[0]["ph_patch"] - out[1]["ph_patch"]).max() <= 1e-9
+
+
+# grids either side of the lines between 4 and 8 warps a block: one round of blocks of
+# 4, one of 8, two of 4, and the padding's share; alone and in window blocks
+@pytest.mark.parametrize("cells,m", [(30, 4), (40, 100), (40, 116), (40, 148), (64, 28), (64, 68), (64, 76)])
+def test_warps_a_block(cuda_lib, cells, m):
+    from pystamps_b200 import stage2 as S
+    from pystamps_b200 import synth
+
+    prep = S.prepare_patch(synth.make_patch(2500, m, cells, 41, seed=390 + m, n_rand=1000), nr=np.ones(100))
+    out = []
+    with S.Stage2Context() as c:
+        c.load(prep)
+        for warps, form in ((0, 0), (4, 0), (8, 0), (0, 1)):
+            c.launch_shapes([0, warps, 0, 0, form])
+            c.reset()
+            c.iterate(1)
+            out.append(c.download(["ph_patch"])["ph_patch"])
+    for o in out[1:]:
+        np.testing.assert_array_equal(o, out[0])
