@@ -93,7 +93,7 @@ __device__ __forceinline__ void compute_f(const ClapArgs& a, const int ix1, cons
   int li = static_cast<int>((static_cast<uint32_t>(pix0) * inv_nw) >> 16), lj = pix0 - li * nw;
   // columns M .. Mp - 1 of the grid are zero, c is even and Mp a multiple of 4
   const float2* src = grid + (static_cast<int64_t>(i1) * a.n_j + j1) * a.Mp + c;
-  const int row = a.n_j * a.Mp;  // 24 or more rows of 8-byte cells fit in memory: < 2^31
+  const int row = a.n_j * a.Mp;  // the window stack, 16 cells or more a grid cell, fits in memory: < 2^31
   const int pix_end = c < a.Mp ? nw2 : 0;
   float* re0 = &m.tiles[q].re[0][0];
   constexpr int kIm = 32 * kTileRow, kNext = sizeof(m.tiles[0]) / sizeof(float);  // tile q's im, tile q + 1
@@ -104,8 +104,8 @@ __device__ __forceinline__ void compute_f(const ClapArgs& a, const int ix1, cons
     for (int u = 0; u < kLoadU; ++u) {
       v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
       at[u] = li * kTileRow + lj;
-      // an address per access from li and lj: with one pointer stepped along, the
-      // compiler took it as the same for all lanes in the <4, 24, true> instance
+      // an address per access from li and lj: with one pointer stepped along to the same
+      // addresses, the <4, 24, true> instance read other cells (cause not found)
       if (p0 + u * (NT / NQ) < pix_end)
         v[u] = *reinterpret_cast<const float4*>(src + (static_cast<int64_t>(li) * row + lj * a.Mp));
       li += dli;

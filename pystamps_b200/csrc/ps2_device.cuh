@@ -15,13 +15,6 @@ constexpr int kCohBins = 100;
 // each product separately (Rust never contracts a*b+c into an FMA); the
 // topofit trial sweep, which the reference does not share bit-for-bit anyway,
 // uses plain (contractible) arithmetic.
-struct c32 {
-  float x, y;
-};
-struct c64d {
-  double x, y;
-};
-
 __device__ __forceinline__ float2 cmul_rn(float2 a, float2 b) {
   // (a.re*b.re - a.im*b.im, a.re*b.im + a.im*b.re) with every product rounded
   return make_float2(__fsub_rn(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y)),

@@ -201,50 +201,6 @@ cudaError_t launch_bin(const BinArgs& a, bool fp64, int sm_count, cudaStream_t s
   return cudaGetLastError();
 }
 
-// ====================================================================== FFT
-// Radix-2 decimation-in-time FFT of 32 points held in registers (textbook
-// Cooley-Tukey). Forward uses e^{-2 pi i k/32}; inverse the conjugate and no
-// scaling (the 1/1024 is folded into the overlap-add weight, like rustfft's
-// unnormalised inverse followed by inv_scale in the reference).
-template <typename R, bool INV>
-__device__ __forceinline__ void fft32(typename CT<R>::C (&x)[32], const typename CT<R>::Tw& tw) {
-  using C = typename CT<R>::C;
-#pragma unroll
-  for (int i = 0; i < 32; ++i) {
-    const int r = ((i & 1) << 4) | ((i & 2) << 2) | (i & 4) | ((i & 8) >> 2) | ((i & 16) >> 4);
-    if (r > i) {
-      C t = x[i];
-      x[i] = x[r];
-      x[r] = t;
-    }
-  }
-#pragma unroll
-  for (int half = 1; half < 32; half <<= 1) {
-    const int step = 16 / half;
-#pragma unroll
-    for (int s = 0; s < 32; s += 2 * half) {
-#pragma unroll
-      for (int k = 0; k < half; ++k) {
-        const int ti = k * step;
-        const C u = x[s + k];
-        const C v = x[s + k + half];
-        C t;
-        if (ti == 0) {
-          t = v;
-        } else if (ti == 8) {
-          t = INV ? mk(-v.y, v.x) : mk(v.y, -v.x);
-        } else {
-          C w = tw.w[ti];
-          if (INV) w.y = -w.y;
-          t = cmul(v, w);
-        }
-        x[s + k] = mk(u.x + t.x, u.y + t.y);
-        x[s + k + half] = mk(u.x - t.x, u.y - t.y);
-      }
-    }
-  }
-}
-
 // ================================================================== CLAP ==
 // One warp's 32x32 working set (33-column rows avoid bank conflicts along
 // columns). PAD staggers consecutive tiles: 8 floats for 4 tiles per block, 4
@@ -401,8 +357,10 @@ __device__ __forceinline__ R warp_median1024_pair(const R (&o)[32], R* scratch, 
 // (lane = column) of the tile, in place. The direction is a template parameter
 // (every shared-memory access then has one address form); not inlined: the
 // window code calls it four times and two copies keep the kernel inside the
-// instruction cache.
-// tw holds e^{-2 pi i k/32} (forward) or its conjugate (inverse), k < 16.
+// instruction cache. Radix-2 decimation in time (textbook Cooley-Tukey).
+// tw holds e^{-2 pi i k/32} (forward) or its conjugate (inverse, no scaling: the
+// 1/1024 is folded into the overlap-add weight, like rustfft's unnormalised inverse
+// followed by inv_scale in the reference), k < 16.
 template <typename R, bool rows, int NZ = 32>
 __device__ __noinline__ void fft_pass_t(R (*re)[33], R (*im)[33], const typename CT<R>::C* tw, const int lane) {
   using C = typename CT<R>::C;
@@ -873,8 +831,7 @@ static cudaError_t launch_clap_nw(const ClapArgs& a, const typename CT<R>::Tw& t
   return a.n_win == 24 ? launch_clap_nwin<R, NW, 24>(a, tw, sm_count, st) : launch_clap_nwin<R, NW, 0>(a, tw, sm_count, st);
 }
 
-// FP32 is in clap_f32.cu. Every window's
-// arithmetic is the same whatever the shape.
+// FP32 is in clap_f32.cu. Every window's arithmetic is the same whatever the shape.
 cudaError_t launch_clap(const ClapArgs& a, bool fp64, const Twiddles32d& td, int sm_count, cudaStream_t st) {
   return fp64 ? launch_clap_nw<double, 4>(a, td, sm_count, st) : launch_clap_f32(a, sm_count, st);
 }
@@ -1643,8 +1600,9 @@ __global__ void __launch_bounds__(256) k_trial_phasors(const double* __restrict_
 // reference compares it. The refinement's elementwise steps run over all elements
 // of the R rows, its ordered sums side by side, one lane a chain (by themselves
 // three chains of m dependent additions a row, the whole warp waiting). Bound by
-// the FP64 pipe: 6 operations per (row, trial, column). 300,000 rows x 60 x 161
-// trials: 4.4 -> 2.55 ms.
+// latency: two warps a scheduler (222 registers at R = 8) keep the FP64 pipe 43 %
+// busy with 6 operations per (row, trial, column), issue 41 %. 300,000 rows x 60 x
+// 161 trials: 4.4 -> 2.55 ms.
 constexpr int kHistWarps = 4;
 template <int R>
 __global__ void __launch_bounds__(32 * kHistWarps) k_random_hist(
@@ -1843,7 +1801,7 @@ cudaError_t launch_random_hist(const double* rnd, int64_t n_rand, const double* 
   const int64_t n_ph = static_cast<int64_t>(m) * (2 * n_half + 1);
   k_trial_phasors<<<static_cast<unsigned>(std::min<int64_t>((n_ph + 255) / 256, static_cast<int64_t>(sm_count) * 8)),
                     256, 0, st>>>(bp, m, n_half, phasors);
-  // 8 rows a warp up to 64 columns (four blocks an SM), 4 beyond
+  // 8 rows a warp up to 64 columns (46 KB at 60; registers allow two blocks an SM), 4 beyond
   return m <= 64 ? random_hist_rows<8>(rnd, n_rand, bp, m, ia, ib, small_baseline, n_half, cutoff0, dbin, phasors, hist,
                                        sm_count, st)
                  : random_hist_rows<4>(rnd, n_rand, bp, m, ia, ib, small_baseline, n_half, cutoff0, dbin, phasors, hist,
